@@ -40,6 +40,7 @@ template <class P> struct FluxArgs {
   P *et1[3];           // E_{t1} on faces of each direction (e2x1, e3x2, e1x3)
   int flatten, low_mach;
   double lhlld_phi;
+  P rgm1;              // 1 / (gamma - 1), rounded once
   // inclusive face ranges per direction: lo[dir][0..2] = (k, j, i)
   int lo[3][3], hi[3][3];
   int active[3];
@@ -308,27 +309,60 @@ template <int RE, class P> struct WindowStencil {
 
 // ---------------------------------------------------------------------------------------
 // Face work: Riemann solve of the face `lf` (between cells lf - stride and lf).
-// b_n: the face-normal field of the face (a sweep that prefetched it passes it in).
-template <int S, class P>
-CHQ_D void face_flux(const FluxArgs<P> &A, const DirView<P> &V, int lf, const P wl[8], const P wr[8], const P b_n) {
+//
+// What bounds it: FP64 issue (61 % of the FP64 pipe's cycles in the y/z launch, 71 % in the x
+// launch at 128^3). With compiled divisions and branching limiters a face took 2200 warp
+// instructions at 24 of 32 active lanes and waited on instruction fetch; with chq_quot.cuh and
+// selects it takes 1760, and the FP64 PPM + HLLD flux launch went from 0.880 to 0.539 ms at
+// 128^3 (blast), 5.21 to 3.54 ms at 256^3 (mixed: 2.88 to 2.09 ms), WENO-Z from 1.92 to 0.96 ms
+// at 128^3, OT 256^2 from 43 to 22 us.
+
+// low-Mach blend of the normal velocities, Thornber et al. (2008) (src/physics.hpp:170-178)
+template <class P> CHQ_D void low_mach_blend(MState<P> &L, MState<P> &R, P cl, P cr) {
+  const P z = fmin_(P(1), fmax_(divz(fabs_(L.u), cl), divz(fabs_(R.u), cr)));
+  const P um = P(0.5) * (L.u + R.u), ud = P(0.5) * (z * (L.u - R.u));
+  L.u = um + ud;
+  R.u = um - ud;
+}
+
+// The face solved again from memory with plain divisions (hlld), for the rare face whose
+// divisors leave the range of hlld_q: both cells' states by the per-cell reconstruction, which
+// gives the sweeps' states bit for bit. Not inlined and given nothing but the face's place, so
+// that the hot code keeps none of its operands alive for it.
+template <int R, int S, bool CHAR, class P>
+__device__ __noinline__ void face_plain(const FluxArgs<P> *args, int d, int lf);
+
+// Solver only; b_n: the face-normal field of the face. PLAIN: hlld with plain divisions.
+// Returns false when hlld_q's divisors left their range (f is then undefined).
+template <int S, bool PLAIN, class P>
+CHQ_D bool face_solve(const FluxArgs<P> &A, const DirView<P> &V, int lf, const P wl[8], const P wr[8], const P b_n, P f[NFLX]) {
   const P gamma = P(A.eos.gamma), gm1 = P(A.eos.gm1);
   MState<P> L{wl[0], wl[1], wl[2], wl[3], wl[4], wl[5], wl[6]};
   MState<P> R{wr[0], wr[1], wr[2], wr[3], wr[4], wr[5], wr[6]};
-  if (A.low_mach) {
-    // Thornber et al. (2008) blend of the normal velocities (src/physics.hpp:170-178)
-    const P cl = fast_speed(L, b_n, gamma), cr = fast_speed(R, b_n, gamma);
-    const P z = fmin_(P(1), fmax_(divz(fabs_(L.u), cl), divz(fabs_(R.u), cr)));
-    const P um = P(0.5) * (L.u + R.u), ud = P(0.5) * (z * (L.u - R.u));
-    L.u = um + ud;
-    R.u = um - ud;
+  if constexpr (S == S_HLLE) {
+    if (A.low_mach) low_mach_blend(L, R, fast_speed(L, b_n, gamma), fast_speed(R, b_n, gamma));
+    hlle(L, R, b_n, gamma, gm1, f);
+    return true;
   }
-  P f[NFLX];
+  const P bnsq = b_n * b_n;
+  const P bsql = bnsq + L.by * L.by + L.bz * L.bz, bsqr = bnsq + R.by * R.by + R.bz * R.bz;
+  bool ok = true;
+  P cl, cr;
+  if constexpr (PLAIN) {
+    cl = fast_speed(L, b_n, gamma);
+    cr = fast_speed(R, b_n, gamma);
+  } else {
+    cl = fast_speed_q(L, b_n, bsql, gamma, ok);
+    cr = fast_speed_q(R, b_n, bsqr, gamma, ok);
+  }
+  if (A.low_mach) low_mach_blend(L, R, cl, cr);
   if constexpr (S == S_HLLD) {
-    hlld<false>(L, R, b_n, gamma, gm1, f, P(1), P(1));
+    if constexpr (PLAIN) hlld<false>(L, R, b_n, gamma, gm1, f, P(1), P(1));
+    else ok = hlld_q<false>(L, R, b_n, gm1, A.rgm1, bsql, bsqr, cl, cr, P(1), P(1), f) && ok;
   } else if constexpr (S == S_LHLLD) {
     // shock detector theta and low-Mach factor phi (src/physics.hpp:183-211)
     const int lL = lf - V.st;
-    const P cfmax = fmax_(fast_speed(L, b_n, gamma), fast_speed(R, b_n, gamma));
+    const P cfmax = fmax_(cl, cr);
     const P *wu = V.src[1], *wv = V.src[2], *ww = V.src[3];
     const int s1 = V.s1, s2 = V.s2;
     const P du = ldg(wu + lf) - ldg(wu + lL);
@@ -343,29 +377,61 @@ CHQ_D void face_flux(const FluxArgs<P> &A, const DirView<P> &V, int lf, const P 
                          fmin_(ldg(ww + lf) - ldg(ww + lf - s2), ldg(ww + lf + s2) - ldg(ww + lf)));
       dvw = fmin_(dvw, d2);
     }
-    const P ratio = fmin_(P(1), (-fmin_(du, P(0)) + cfmax) / (-dvw + cfmax));
+    const P num = -fmin_(du, P(0)) + cfmax, den = -dvw + cfmax;
+    P ratio, chi;
+    if constexpr (PLAIN) {
+      ratio = num / den;
+      chi = divz(fmax_(flow_speed_u(L, b_n), flow_speed_u(R, b_n)), cfmax);
+    } else {
+      ok = ok && in_range(den) && in_range(cfmax);
+      ratio = quot(num, den, rcp_a(den));
+      chi = quot(fmax_(flow_speed_q(L, b_n), flow_speed_q(R, b_n)), cfmax, rcp_a(cfmax));
+    }
+    ratio = fmin_(P(1), ratio);
+    chi = fmin_(P(1), chi);
     const P r2 = ratio * ratio;
     const P theta = r2 * r2;
-    const P chi = fmin_(P(1), divz(fmax_(flow_speed_u(L, b_n), flow_speed_u(R, b_n)), cfmax));
     const P phi = (A.lhlld_phi >= 0.0) ? P(A.lhlld_phi) : chi * (P(2) - chi);
-    hlld<true>(L, R, b_n, gamma, gm1, f, theta, phi);
-  } else {
-    hlle(L, R, b_n, gamma, gm1, f);
+    if constexpr (PLAIN) hlld<true>(L, R, b_n, gamma, gm1, f, theta, phi);
+    else ok = hlld_q<true>(L, R, b_n, gm1, A.rgm1, bsql, bsqr, cl, cr, theta, phi, f) && ok;
   }
+  return ok;
+}
+
+// the face's outputs from its fluxes
+template <class P>
+CHQ_D void face_store(const DirView<P> &V, int lf, const P f[NFLX], P sl, P sr) {
   V.out[0][lf] = f[FD];
   V.out[1][lf] = f[FMU];
   V.out[2][lf] = f[FMV];
   V.out[3][lf] = f[FMW];
   V.out[4][lf] = f[FEN];
   // entropy flux upwinded with the mass flux, averaged at an exact zero
-  const P sl = wl[7], sr = wr[7];
   V.out[5][lf] = (f[FD] > P(0)) ? f[FD] * sl : (f[FD] < P(0)) ? f[FD] * sr : P(0.5) * (f[FD] * (sl + sr));
   V.out[6][lf] = -f[FBY];
   V.out[7][lf] = f[FBZ];
 }
-template <int S, class P>
-CHQ_D void face_flux(const FluxArgs<P> &A, const DirView<P> &V, int lf, const P wl[8], const P wr[8]) {
-  face_flux<S, P>(A, V, lf, wl, wr, P(V.bn[lf]));
+
+// d: the direction of the view
+template <int R, int S, bool CHAR, class P>
+CHQ_D void face_flux(const FluxArgs<P> &A, const DirView<P> &V, int d, int lf, const P wl[8], const P wr[8], const P b_n) {
+  P f[NFLX];
+  const bool ok = face_solve<S, false, P>(A, V, lf, wl, wr, b_n, f);
+  face_store<P>(V, lf, f, wl[7], wr[7]);
+  if constexpr (S != S_HLLE) {
+    if (!ok) face_plain<R, S, CHAR, P>(&A, d, lf);
+  }
+}
+
+template <int R, int S, bool CHAR, class P>
+__device__ __noinline__ void face_plain(const FluxArgs<P> *args, int d, int lf) {
+  const FluxArgs<P> &A = *args;
+  const DirView<P> V = dir_view(A, d);
+  P aL[8], aR[8], wl[8], f[NFLX];
+  cell_states<R, CHAR, P>(A, V, lf - V.st, aL, wl);
+  cell_states<R, CHAR, P>(A, V, lf, aL, aR);
+  face_solve<S, true, P>(A, V, lf, wl, aL, P(V.bn[lf]), f);
+  face_store<P>(V, lf, f, wl[7], aL[7]);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -390,7 +456,7 @@ CHQ_D void sweep_x(const FluxArgs<P> &A, int wid) {
   P wl[8];
 #pragma unroll
   for (int n = 0; n < 8; ++n) wl[n] = __shfl_up_sync(0xffffffffu, aR[n], 1);
-  if (have && lane > 0) face_flux<S, P>(A, V, lc, wl, aL, bnf);
+  if (have && lane > 0) face_flux<R, S, CHAR, P>(A, V, 0, lc, wl, aL, bnf);
 }
 
 // Faces per x-sweep warp: 31 in the per-cell form (lane 0 contributes only its right state),
@@ -439,9 +505,9 @@ CHQ_D void sweep_x_ppm(const FluxArgs<P> &A, int wid) {
 #pragma unroll
   for (int n = 0; n < 8; ++n) {
     const P qm = QM[n], q0 = Q0[n], qp = QP[n];
-    const P sc = mc_slope(qm, q0, qp);
+    const P sc = mc_slope2(qm, q0, qp);
     const P sp = __shfl_down_sync(0xffffffffu, sc, 1);    // s_{c+1}
-    const P fp = ppm_face(q0, qp, sc, sp);                 // F_{c+1/2}, unlimited
+    const P fp = ppm_face2(q0, qp, sc, sp);                 // F_{c+1/2}, unlimited
     P l = __shfl_up_sync(0xffffffffu, fp, 1), r = fp;     // F_{c-1/2}
     ppm_limit(q0, l, r);
     aL[n] = l;
@@ -454,7 +520,7 @@ CHQ_D void sweep_x_ppm(const FluxArgs<P> &A, int wid) {
   P wl[8];
 #pragma unroll
   for (int n = 0; n < 8; ++n) wl[n] = __shfl_up_sync(0xffffffffu, aR[n], 1);
-  if (lane >= 2 && lane <= 30 && c <= A.hi[0][2]) face_flux<S, P>(A, V, base + c, wl, aL, bnf);
+  if (lane >= 2 && lane <= 30 && c <= A.hi[0][2]) face_flux<R_PPM, S, false, P>(A, V, 0, base + c, wl, aL, bnf);
 }
 
 // Streaming PPM along a y/z march. Each thread's shared-memory column keeps, per quantity,
@@ -536,11 +602,11 @@ CHQ_D void sweep_yz_ppm(const FluxArgs<P> &A, int d, int wid, P *park, P *win, c
   for (int n = 0; n < 8; ++n) {
     const P *src = V.src[n] + lc;
     const P qm2 = ldg(src - 2 * st), qm1 = ldg(src - st), q0 = ldg(src), qp1 = ldg(src + st);
-    const P sm = mc_slope(qm2, qm1, q0), sc = mc_slope(qm1, q0, qp1);
+    const P sm = mc_slope2(qm2, qm1, q0), sc = mc_slope2(qm1, q0, qp1);
     CHQ_SLOT(n, Q0) = q0;
     CHQ_SLOT(n, Q1) = qp1;
     CHQ_SLOT(n, S) = sc;
-    CHQ_SLOT(n, F) = ppm_face(qm1, q0, sm, sc);
+    CHQ_SLOT(n, F) = ppm_face2(qm1, q0, sm, sc);
     if (n == 1) CHQ_SLOT(1, X1) = qm1;
     if (n == 4) {
       CHQ_SLOT(4, X1) = qm2;
@@ -577,8 +643,8 @@ CHQ_D void sweep_yz_ppm(const FluxArgs<P> &A, int d, int wid, P *park, P *win, c
     for (int n = 0; n < 8; ++n) {
       const P q0 = CHQ_SLOT(n, Q0), q1 = CHQ_SLOT(n, Q1), q2 = CHQ_SLOT(n, Q2);
       const P sc = CHQ_SLOT(n, S), fm = CHQ_SLOT(n, F);
-      const P sp = mc_slope(q0, q1, q2);          // s_{c+1}
-      const P fp = ppm_face(q0, q1, sc, sp);      // F_{c+1/2}, unlimited
+      const P sp = mc_slope2(q0, q1, q2);          // s_{c+1}
+      const P fp = ppm_face2(q0, q1, sc, sp);      // F_{c+1/2}, unlimited
       P l = fm, r = fp;
       ppm_limit(q0, l, r);
       aL[n] = l;
@@ -620,8 +686,7 @@ CHQ_D void sweep_yz_ppm(const FluxArgs<P> &A, int d, int wid, P *park, P *win, c
 #pragma unroll
     for (int n = 0; n < 8; ++n) park[n * kYzThreads + t] = aR[n];
     if (f >= f0) {
-      if constexpr (PFB) face_flux<S, P>(A, V, lc, wl, aL, bnv);
-      else face_flux<S, P>(A, V, lc, wl, aL);
+      face_flux<R_PPM, S, false, P>(A, V, d, lc, wl, aL, PFB ? bnv : P(V.bn[lc]));
     }
 #pragma unroll
     for (int n = 0; n < 8; ++n) wl[n] = park[n * kYzThreads + t];
@@ -697,8 +762,7 @@ CHQ_D void sweep_yz(const FluxArgs<P> &A, int d, int wid, P *park, P *win) {
 #pragma unroll
     for (int n = 0; n < 8; ++n) park[n * kYzThreads + t] = aR[n];
     if (f >= f0) {
-      if constexpr (PFB) face_flux<S, P>(A, V, lc, wl, aL, bnv);
-      else face_flux<S, P>(A, V, lc, wl, aL);
+      face_flux<R, S, CHAR, P>(A, V, d, lc, wl, aL, PFB ? bnv : P(V.bn[lc]));
     }
 #pragma unroll
     for (int n = 0; n < 8; ++n) wl[n] = park[n * kYzThreads + t];
@@ -706,14 +770,17 @@ CHQ_D void sweep_yz(const FluxArgs<P> &A, int d, int wid, P *park, P *win) {
 }
 
 // Resident 128-thread blocks per SM the x-sweep kernel is compiled for (register cap), in two
-// variants that the autotuner chooses between per scheme, precision and mesh: V = 0 at 5
-// (FP64, 96 registers) / 10 (FP32, 48 registers) blocks, V = 1 at 6 / 12 blocks (more
-// resident warps to hide the FP64 / FP32 latency, fewer registers, some spilling to L1).
+// variants that the autotuner chooses between per scheme, precision and mesh: V = 0 at 4
+// (FP64, 128 registers) / 8 (FP32, 64 registers) blocks, V = 1 at 5 / 10 blocks (more resident
+// warps, fewer registers, some spilling to L1). Since the solver has no branches its two sides
+// and the quantities interleave, so registers hide more latency than warps do: FP64 PPM flux
+// launches at 256^3 measured 3.86 ms with 5 blocks and 3.77 ms with 4 (3: 3.70 against 3.54 in
+// the final build), the mixed form 2.18 / 2.13 ms with 10 / 8.
 #ifndef CHQ_FLUX_MINB_D
-#define CHQ_FLUX_MINB_D 5
+#define CHQ_FLUX_MINB_D 4
 #endif
 #ifndef CHQ_FLUX_MINB_F
-#define CHQ_FLUX_MINB_F 10
+#define CHQ_FLUX_MINB_F 8
 #endif
 template <class P, int V = 0> struct FluxMinBlocks {
   static constexpr int v = (sizeof(P) == 8) ? CHQ_FLUX_MINB_D + V : CHQ_FLUX_MINB_F + 2 * V;
@@ -722,12 +789,13 @@ constexpr int kFluxXVariants = 2;
 
 // Single-mesh launches split by sweep: the x-sweep kernel needs no shared window, so it keeps
 // the full L1 and the register cap above; the y/z kernel holds 8 + 8(2RE+1) shared columns
-// per thread (48 KB per block in FP64 PPM / PPMX / WENO-Z), which sets its residency.
+// per thread (53 KB per block in FP64 PPM). 3 blocks (168 registers) beat 4 (128 registers) by
+// 6 % and 2 by 9 % in FP64 PPM at 256^3, although 4 would fit: see the x sweep's caps.
 #ifndef CHQ_FLUXYZ_MINB_D
-#define CHQ_FLUXYZ_MINB_D 4
+#define CHQ_FLUXYZ_MINB_D 3
 #endif
 #ifndef CHQ_FLUXYZ_MINB_F
-#define CHQ_FLUXYZ_MINB_F 8
+#define CHQ_FLUXYZ_MINB_F 6
 #endif
 template <class P> struct FluxYzMinBlocks { static constexpr int v = (sizeof(P) == 8) ? CHQ_FLUXYZ_MINB_D : CHQ_FLUXYZ_MINB_F; };
 
@@ -740,7 +808,7 @@ template <int R, class P> __host__ __device__ constexpr size_t flux_yz_smem() {
 }
 
 template <int R, int S, bool CHAR, class P, int V = 0>
-__global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_kernel(const FluxArgs<P> A) {
+__global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_kernel(const __grid_constant__ FluxArgs<P> A) {
   if (A.skip && *A.skip) return;
   const int wid = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 5);
   if (wid < (int)A.nwarp[0]) {
@@ -750,7 +818,7 @@ __global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_kernel(c
 }
 
 template <int R, int S, bool CHAR, class P>
-__global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<P>::v) flux_yz_kernel(const FluxArgs<P> A) {
+__global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<P>::v) flux_yz_kernel(const __grid_constant__ FluxArgs<P> A) {
   extern __shared__ __align__(16) unsigned char flux_dsm[];
   P *park = reinterpret_cast<P *>(flux_dsm);
   P *win = park + 8 * kYzThreads;

@@ -391,6 +391,7 @@ FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask) {
   a.flatten = m->cfg.flatten;
   a.low_mach = m->cfg.low_mach;
   a.lhlld_phi = m->cfg.lhlld_phi;
+  a.rgm1 = P(1) / P(m->eos.gm1);
   a.seglen = m->seglen;
   a.xvar = m->xvar;
   a.yzvar = m->tma_ok ? m->yzvar : 0;

@@ -12,6 +12,7 @@
 // 0 mass, 1 normal momentum, 2/3 transverse momenta, 4 energy, 5/6 transverse fields.
 #pragma once
 #include "chq_common.cuh"
+#include "chq_quot.cuh"
 
 namespace chq {
 
@@ -297,6 +298,182 @@ CHQ_HD void hlld(const MState<T> &L, const MState<T> &R, T bn, T gamma, T gm1, T
 #pragma unroll
     for (int n = 0; n < NFLX; ++n) f[n] = T(0.5) * (f[n] + fb[n]);
   }
+}
+
+// ---------------------------------------------------------------------------------------
+// The face solver of the flux kernel: hlld with the quotients of chq_quot.cuh. Bound by FP64
+// issue, so it evaluates only what the selected side needs: both sides' speeds and star
+// states, then the energies and the flux of one side. Every rounded operation has hlld's
+// operands, so the fluxes are the same; `ok` turns false when a divisor leaves the range the
+// quotients are exact in (vacuum, non-finite states, a degenerate negative star denominator),
+// and the caller then evaluates hlld itself.
+
+// fast magnetosonic speed (fast_speed) from bsq = B^2
+template <class T> CHQ_D T fast_speed_q(const MState<T> &s, T bn, T bsq, T gamma, bool &ok) {
+  const T gp = gamma * s.p;
+  const T yd = rcp_a(s.d);
+  const T a = quot(gp + bsq, s.d, yd);
+  const T dd = s.d * s.d;
+  const T disc = a * a - quot(T(4) * gp * bn * bn, dd, yd * yd);
+  const T root = sqrt_q(disc);
+  ok = ok && in_range(s.d) && in_range(a);
+  return sqrt_q(T(0.5) * (a + (disc > RootFloor<T>::v ? root : T(0))));
+}
+
+// modified fast speed of LHLLD (flow_speed_u)
+template <class T> CHQ_D T flow_speed_q(const MState<T> &s, T bn) {
+  const T vsq = s.u * s.u + s.v * s.v + s.w * s.w;
+  const T yd = rcp_a(s.d);
+  const T casq = quot(bn * bn + s.by * s.by + s.bz * s.bz, s.d, yd);
+  const T caxsq = quot(bn * bn, s.d, yd);
+  const T a = casq + vsq;
+  const T disc = a * a - T(4) * vsq * caxsq;
+  const T root = sqrt_q(disc);
+  const T h = T(0.5) * (a + (disc > RootFloor<T>::v ? root : T(0)));
+  const T r = sqrt_q(h);
+  return (h > RootFloor<T>::v) ? r : T(0);
+}
+
+// single-star transverse velocity and field of one side (star_side); dm = rho (S - u), sms = S - S_M
+template <class T>
+CHQ_D void star_side_q(const MState<T> &S, T dm, T slm, T sms, T sm, T bn, T bnsq, T &vs, T &ws, T &bys, T &bzs,
+                       bool &ok) {
+  const T t = dm * sms;
+  const T den = t - bnsq;
+  const bool deg = fabs_(den) <= T(1e-12) * (fabs_(t) + bnsq) + Tiny<T>::v;
+  const T y = rcp_a(den);
+  const T nv = quot(bn * (sm - S.u), den, y);
+  const T nb = quot(dm * slm - bnsq, den, y);
+  vs = deg ? S.v : S.v - S.by * nv;
+  ws = deg ? S.w : S.w - S.bz * nv;
+  bys = deg ? S.by : S.by * nb;
+  bzs = deg ? S.bz : S.bz * nb;
+  ok = ok && (deg || in_range(den));
+}
+
+// total energy (energy_ptot) with the quotient by gamma - 1 taken from its rounded reciprocal
+template <class T> CHQ_D T energy_q(const MState<T> &s, T bsq, T gm1, T rgm1) {
+  const T vsq = s.u * s.u + s.v * s.v + s.w * s.w;
+  return fma_(T(0.5), s.d * vsq + bsq, quot(s.p, gm1, rgm1));
+}
+
+// One side of a star region: the side's state S with its pressure, wave speed s, S - u (slm),
+// star density, star transverse state, |S - S_M| (n) and its reciprocal (y), and what its
+// double-star state adds (ss: the Alfven speed, sqd: sqrt of the star density).
+template <class T> struct StarSide {
+  MState<T> S;
+  T bsq, pt, s, slm, n, y, ds, vs, ws, bys, bzs, sqd, ss;
+};
+
+// single-star (single) or double-star flux of the side
+template <bool LHLLD, class T>
+CHQ_D void star_region_flux(const StarSide<T> &Q, bool left, bool single, T bn, T gm1, T rgm1, T sm, T pts, T vss, T wss,
+                            T byss, T bzss, T f[NFLX]) {
+  const MState<T> &S = Q.S;
+  const T e = energy_q(S, Q.bsq, gm1, rgm1);
+  const T vdotb = (S.u * bn + S.v * S.by) + S.w * S.bz;
+  const T vdotb_s = (sm * bn + Q.vs * Q.bys) + Q.ws * Q.bzs;
+  const T num = ((Q.slm * e - Q.pt * S.u) + pts * sm) + bn * (vdotb - vdotb_s);
+  const T es = quot(left ? -num : num, Q.n, Q.y);
+  const T vdotb_ss = (sm * bn + vss * byss) + wss * bzss;
+  const T t = Q.sqd * flip_sign(vdotb_s - vdotb_ss, bn);
+  const T ess = es + (left ? -t : t);
+  if constexpr (LHLLD) {
+    star_flux(Q.ds, sm, single ? Q.vs : vss, single ? Q.ws : wss, single ? es : ess, single ? Q.bys : byss,
+              single ? Q.bzs : bzss, bn, pts, f);
+  } else {
+    flux_from(S, bn, e, Q.pt, f);
+    const T us[NFLX] = {Q.ds, Q.ds * sm, Q.ds * Q.vs, Q.ds * Q.ws, es, Q.bys, Q.bzs};
+    const T u[NFLX] = {S.d, S.d * S.u, S.d * S.v, S.d * S.w, e, S.by, S.bz};
+#pragma unroll
+    for (int n = 0; n < NFLX; ++n) f[n] = f[n] + Q.s * (us[n] - u[n]);
+    if (!single) {
+      // the double star keeps the star density and normal momentum: those differences are zero
+      const T uss[NFLX] = {Q.ds, Q.ds * sm, Q.ds * vss, Q.ds * wss, ess, byss, bzss};
+#pragma unroll
+      for (int n = FMV; n < NFLX; ++n) f[n] = f[n] + Q.ss * (uss[n] - us[n]);
+    }
+  }
+}
+
+// cl, cr: the sides' fast speeds; bsql, bsqr: their B^2; rgm1 = RN(1 / gm1)
+template <bool LHLLD, class T>
+CHQ_D bool hlld_q(const MState<T> &L, const MState<T> &R, T bn, T gm1, T rgm1, T bsql, T bsqr, T cl, T cr, T theta,
+                  T phi, T f[NFLX]) {
+  const T bnsq = bn * bn;
+  const T ptl = fma_(T(0.5), bsql, L.p), ptr = fma_(T(0.5), bsqr, R.p);
+  T sl, sr;
+  if constexpr (LHLLD) {
+    const T cmax = (cl > cr) ? cl : cr;
+    const T ul = ((L.u < R.u) ? L.u : R.u) - cmax, ur = ((L.u > R.u) ? L.u : R.u) + cmax;
+    sl = (ul < T(0)) ? ul : T(0);
+    sr = (ur > T(0)) ? ur : T(0);
+  } else {
+    const T a = L.u - cl, b = R.u - cr, c = L.u + cl, d = R.u + cr;
+    sl = (a < b) ? a : b;
+    sr = (c > d) ? c : d;
+  }
+  if (sl >= T(0) || sr <= T(0)) {
+    const bool left = sl >= T(0);
+    const MState<T> S{left ? L.d : R.d, left ? L.u : R.u, left ? L.v : R.v, left ? L.w : R.w,
+                      left ? L.p : R.p, left ? L.by : R.by, left ? L.bz : R.bz};
+    flux_from(S, bn, energy_q(S, left ? bsql : bsqr, gm1, rgm1), left ? ptl : ptr, f);
+    return true;
+  }
+  const T slml = sl - L.u, srmr = sr - R.u;
+  const T dsl = L.d * slml, dsr = R.d * srmr;
+  const T dds = dsr - dsl;
+  const T iden = rcp_rn(dds);
+  const T sm = ((dsr * R.u - dsl * L.u) + theta * (ptl - ptr)) * iden;
+  const T pts = ((dsr * ptl - dsl * ptr) + (phi * ((L.d * R.d) * (srmr * slml))) * (R.u - L.u)) * iden;
+  // left divisors negated (S_M - S_L > 0), which negates the numerators: the same quotients
+  const T nl = sm - sl, nr = sr - sm;
+  const T yl = rcp_a(nl), yr = rcp_a(nr);
+  const T dls = quot(-dsl, nl, yl), drs = quot(dsr, nr, yr);
+  bool ok = in_range(dds) && in_range(nl) && in_range(nr) && in_range(dls) && in_range(drs);
+  T yql, yqr;
+  const T sqdl = sqrt_q(dls, yql), sqdr = sqrt_q(drs, yqr);
+  const T abn = fabs_(bn);
+  const T sls = sm - quot(abn, sqdl, yql);
+  const T srs = sm + quot(abn, sqdr, yqr);
+  // region and side as in hlld
+  const bool star_l = sls > T(0);
+  const bool star_r = !star_l && (srs < T(0));
+  const bool single = star_l || star_r || (bnsq <= T(1e-12) * (ptl + ptr));
+  const bool pos = sm > T(0), neg = sm < T(0);
+  const bool both = !star_l && !star_r && !pos && !neg;
+  const bool left = star_l || (!star_r && (pos || both));
+  T vls, wls, byls, bzls, vrs, wrs, byrs, bzrs;
+  star_side_q(L, dsl, slml, -nl, sm, bn, bnsq, vls, wls, byls, bzls, ok);
+  star_side_q(R, dsr, srmr, nr, sm, bn, bnsq, vrs, wrs, byrs, bzrs, ok);
+  T vss = T(0), wss = T(0), byss = T(0), bzss = T(0);
+  if (!single) {
+    const T inv = rcp_rn(sqdl + sqdr);
+    vss = ((sqdl * vls + sqdr * vrs) + flip_sign(byrs - byls, bn)) * inv;
+    wss = ((sqdl * wls + sqdr * wrs) + flip_sign(bzrs - bzls, bn)) * inv;
+    byss = ((sqdl * byrs + sqdr * byls) + (sqdl * sqdr) * flip_sign(vrs - vls, bn)) * inv;
+    bzss = ((sqdl * bzrs + sqdr * bzls) + (sqdl * sqdr) * flip_sign(wrs - wls, bn)) * inv;
+  }
+  // a contact that stands exactly still (gas at rest): the mean of both sides' fluxes; the
+  // right side's is evaluated here, where its operands are still at hand
+  T f0[NFLX];
+#pragma unroll
+  for (int n = 0; n < NFLX; ++n) f0[n] = T(0);
+  if (both) {
+    const StarSide<T> Q{R, bsqr, ptr, sr, srmr, nr, yr, drs, vrs, wrs, byrs, bzrs, sqdr, srs};
+    star_region_flux<LHLLD>(Q, false, single, bn, gm1, rgm1, sm, pts, vss, wss, byss, bzss, f0);
+  }
+  const StarSide<T> Q{{left ? L.d : R.d, left ? L.u : R.u, left ? L.v : R.v, left ? L.w : R.w,
+                       left ? L.p : R.p, left ? L.by : R.by, left ? L.bz : R.bz},
+                      left ? bsql : bsqr, left ? ptl : ptr, left ? sl : sr, left ? slml : srmr, left ? nl : nr,
+                      left ? yl : yr, left ? dls : drs, left ? vls : vrs, left ? wls : wrs, left ? byls : byrs,
+                      left ? bzls : bzrs, left ? sqdl : sqdr, left ? sls : srs};
+  star_region_flux<LHLLD>(Q, left, single, bn, gm1, rgm1, sm, pts, vss, wss, byss, bzss, f);
+  if (both) {
+#pragma unroll
+    for (int n = 0; n < NFLX; ++n) f[n] = T(0.5) * (f[n] + f0[n]);
+  }
+  return ok;
 }
 
 }  // namespace chq

@@ -221,8 +221,8 @@ CHQ_API int chq_profile(chq_mesh *m, int enable);
  *  - march length = faces each thread of the y/z sweeps carries its cell states across
  *    (CHQ_TUNE_LENGTHS). The default is the longest of 16, 8, 4 that keeps a full device of
  *    y/z threads busy (16 from about 128^3 up, 4 for small meshes);
- *  - x-sweep variant = the register cap the x-sweep kernel is compiled for (0: 5 resident
- *    128-thread blocks per SM in FP64 / 10 in FP32; 1: 6 / 12, more resident warps, fewer
+ *  - x-sweep variant = the register cap the x-sweep kernel is compiled for (0: 4 resident
+ *    128-thread blocks per SM in FP64 / 8 in FP32; 1: 5 / 10, more resident warps, fewer
  *    registers). Default 0. The tuner varies it in the FP64 form only: there both builds
  *    compute the same bits, while in the mixed form the compiler may contract the FP32
  *    arithmetic of the two builds differently (chq_set_xvariant still selects it there).
