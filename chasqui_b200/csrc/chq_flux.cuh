@@ -7,12 +7,12 @@
 // Fluxes<DIR,R,S> (src/physics.hpp:66-226); the left/right face states never leave the SM.
 //
 // Work decomposition, two launches per stage:
-//   flux_x_kernel : one warp = 32 consecutive cells of a row; lane l computes the (aL, aR)
+//   flux_x_kernel : one warp = 32 consecutive cells of the rows laid end to end; lane l computes the (aL, aR)
 //             pair of its cell once (stencil from L1) and receives its left neighbour's aR by
 //             __shfl_up_sync, so a warp emits 31 faces and no cell parabola is evaluated twice
 //             (PPM: slopes and unlimited interface values are shared between lanes too, and a
 //             warp emits 29 faces).
-//   flux_yz_kernel: lanes run along i (fully coalesced rows); each thread marches `seglen`
+//   flux_yz_kernel: lanes run along i, rows end to end (coalesced); each thread marches `slen`
 //             faces along y or z with its stencil in a shared-memory window that cp.async
 //             refills one cell ahead, and parks the previous cell's aR in shared memory
 //             during the Riemann solve (PPM: the march carries each quantity's slope and
@@ -44,10 +44,13 @@ template <class P> struct FluxArgs {
   // inclusive face ranges per direction: lo[dir][0..2] = (k, j, i)
   int lo[3][3], hi[3][3];
   int active[3];
-  int seglen;          // faces per thread along y/z sweeps
-  long nwarp[3];       // warps per direction
-  int nseg[3];         // segments along the sweep (x: XFaces-face segments)
-  int nchunk;          // 32-wide i chunks for y/z sweeps (aligned to i = 0)
+  int slen[3];         // faces per thread along y/z sweeps (at most the march length)
+  int nseg[3];         // march segments per y/z column
+  int ncol[3];         // y/z: columns (i, outer) of the direction, i fastest
+  int nblk[3];         // y/z: blocks of the direction (kYzThreads columns each x segments)
+  int nxent, nxrow;    // x: cells a row contributes (faces + XLead), rows
+  int nxwarp;          // x: warps
+  int nchunk;          // TMA staging: 32-wide i chunks (aligned to i = 0)
   int xvar;            // x-sweep kernel variant (register cap, FluxMinBlocks); picked by the autotuner
   const int *skip;     // optional device flag: nonzero -> kernel returns immediately
   int yzvar;           // y/z staging of the FP64 streaming-PPM march: 0 cp.async, 1 TMA (autotuner)
@@ -287,6 +290,22 @@ CHQ_D void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2
 #endif
 constexpr int kYzThreads = CHQ_FLUXYZ_THREADS;
 
+// Lane mapping of the y/z sweeps: the direction's columns (i, outer index) are numbered with i
+// fastest and a block takes the next kYzThreads of them for one march segment, so a warp may
+// hold the end of one row and the start of the next. Warps cut at 32-cell boundaries of each
+// row left 4 of 32 lanes busy in every last warp (130 columns at 128^3: 5 warps a row, 81 % of
+// the lanes; 66 at 64^2: 3 warps, 69 %).
+template <class P> CHQ_D bool yz_place(const FluxArgs<P> &A, int d, int blk, int &i, int &outer, int &seg) {
+  const int cb = blk / A.nseg[d];
+  seg = blk - cb * A.nseg[d];
+  const int col = cb * kYzThreads + (int)threadIdx.x;
+  if (col >= A.ncol[d]) return false;
+  const int w = A.hi[d][2] - A.lo[d][2] + 1;
+  outer = col / w;
+  i = A.lo[d][2] + (col - outer * w);
+  return true;
+}
+
 // Marching window: one shared-memory column per thread and quantity, 2RE+1 slots. For the
 // current cell c, slots 0..2RE-1 hold q[c-RE .. c+RE-1] and slot 2RE holds q[c+RE], copied
 // asynchronously one step earlier. Reading the stencil shifts the window down by one slot
@@ -435,17 +454,47 @@ __device__ __noinline__ void face_plain(const FluxArgs<P> *args, int d, int lf) 
 }
 
 // ---------------------------------------------------------------------------------------
+// Lane mapping of the x sweep. The rows (k, j) are laid end to end, each with the cells its
+// faces need (nxent = faces + XLead), and a warp takes the next 32 of them, overlapping the
+// warp before by the 32 - XFaces lanes whose states only feed their neighbours. A row end thus
+// costs XLead lanes instead of the rest of a warp: at 128 faces a row 89 % of the lanes emit
+// faces, with warps cut at the row ends it was 81 % (64: 87 and 68 %, 256: 89 and 89 %).
+//
+// Faces per x-sweep warp: 31 in the per-cell form (lane 0 contributes only its right state),
+// 29 in the streaming PPM form (lanes 0 and 31 contribute only their slope and interface
+// value, so the states of lanes 1..30 are complete and lanes 2..30 emit faces). XLead: cells
+// before (XBack) and after a row's faces.
+template <int R, bool CHAR> struct XFaces {
+  static constexpr bool stream = (R == R_PPM && !CHAR);
+  static constexpr int v = stream ? 29 : 31;
+  static constexpr int back = stream ? 2 : 1, lead = stream ? 3 : 1;
+};
+
+// row and cell of this lane's place; false past the last row
+template <class P> CHQ_D bool x_place(const FluxArgs<P> &A, int wid, int per, int back, int &k, int &j, int &c) {
+  const int E = A.nxent, lane = threadIdx.x & 31;
+  const int base = wid * per;
+  int row = base / E;
+  int e = base - row * E + lane;
+  while (e >= E) {
+    e -= E;
+    ++row;
+  }
+  const bool have = row < A.nxrow;
+  row = min(row, A.nxrow - 1);
+  const int nj = A.hi[0][1] - A.lo[0][1] + 1;
+  const int q = row / nj;
+  k = A.lo[0][0] + q;
+  j = A.lo[0][1] + (row - q * nj);
+  c = A.lo[0][2] - back + e;
+  return have;
+}
+
 template <int R, int S, bool CHAR, class P>
 CHQ_D void sweep_x(const FluxArgs<P> &A, int wid) {
-  const int lane = threadIdx.x & 31;
-  const int nseg = A.nseg[0];
-  const int row = wid / nseg;
-  const int seg = (int)(wid - row * nseg);
-  const int nj = A.hi[0][1] - A.lo[0][1] + 1;
-  const int k = A.lo[0][0] + (int)(row / nj);
-  const int j = A.lo[0][1] + (row - (row / nj) * nj);
-  const int c = A.lo[0][2] - 1 + 31 * seg + lane;   // this lane's cell
-  const bool have = (c <= A.hi[0][2]);
+  using X = XFaces<R, CHAR>;
+  int k, j, c;
+  const bool have = x_place(A, wid, X::v, X::back, k, j, c);   // this lane's cell
   const DirView<P> V = dir_view(A, 0);
   P aL[8], aR[8];
 #pragma unroll
@@ -456,13 +505,8 @@ CHQ_D void sweep_x(const FluxArgs<P> &A, int wid) {
   P wl[8];
 #pragma unroll
   for (int n = 0; n < 8; ++n) wl[n] = __shfl_up_sync(0xffffffffu, aR[n], 1);
-  if (have && lane > 0) face_flux<R, S, CHAR, P>(A, V, 0, lc, wl, aL, bnf);
+  if (have && (threadIdx.x & 31) > 0 && c >= A.lo[0][2]) face_flux<R, S, CHAR, P>(A, V, 0, lc, wl, aL, bnf);
 }
-
-// Faces per x-sweep warp: 31 in the per-cell form (lane 0 contributes only its right state),
-// 29 in the streaming PPM form below (lanes 0 and 31 contribute only their slope and interface
-// value, so the states of lanes 1..30 are complete and lanes 2..30 emit faces).
-template <int R, bool CHAR> struct XFaces { static constexpr int v = (R == R_PPM && !CHAR) ? 29 : 31; };
 
 // Streaming PPM (CW84, src/recon.hpp:21-78) along a row of 32 cells, one per lane. The
 // reference evaluates, for face i, the limited parabolas of cells i-1 and i from their
@@ -473,14 +517,10 @@ template <int R, bool CHAR> struct XFaces { static constexpr int v = (R == R_PPM
 // every expression are the reference's, so the limited states are bitwise the same.
 template <int S, class P>
 CHQ_D void sweep_x_ppm(const FluxArgs<P> &A, int wid) {
+  using X = XFaces<R_PPM, false>;
   const int lane = threadIdx.x & 31;
-  const int nseg = A.nseg[0];
-  const int row = wid / nseg;
-  const int seg = (int)(wid - row * nseg);
-  const int nj = A.hi[0][1] - A.lo[0][1] + 1;
-  const int k = A.lo[0][0] + (int)(row / nj);
-  const int j = A.lo[0][1] + (row - (row / nj) * nj);
-  const int c = A.lo[0][2] - 2 + 29 * seg + lane;   // this lane's cell
+  int k, j, c;
+  const bool have = x_place(A, wid, X::v, X::back, k, j, c);   // this lane's cell
   // lanes past the row's last face (and lane 0's stencil at the row start) read clamped
   // indices inside the row; their states are never used
   const int last = A.g.ni - 1;
@@ -520,7 +560,7 @@ CHQ_D void sweep_x_ppm(const FluxArgs<P> &A, int wid) {
   P wl[8];
 #pragma unroll
   for (int n = 0; n < 8; ++n) wl[n] = __shfl_up_sync(0xffffffffu, aR[n], 1);
-  if (lane >= 2 && lane <= 30 && c <= A.hi[0][2]) face_flux<R_PPM, S, false, P>(A, V, 0, base + c, wl, aL, bnf);
+  if (have && lane >= 2 && lane <= 30 && c >= A.lo[0][2] && c <= A.hi[0][2]) face_flux<R_PPM, S, false, P>(A, V, 0, base + c, wl, aL, bnf);
 }
 
 // Streaming PPM along a y/z march. Each thread's shared-memory column keeps, per quantity,
@@ -546,28 +586,29 @@ struct PpmWin {
 // waits on its mbarrier's phase. Same slots, same values: the states are bitwise those of the
 // cp.async form.
 template <int S, class P, bool TMA = false>
-CHQ_D void sweep_yz_ppm(const FluxArgs<P> &A, int d, int wid, P *park, P *win, const YzMaps *maps = nullptr,
+CHQ_D void sweep_yz_ppm(const FluxArgs<P> &A, int d, int blk, P *park, P *win, const YzMaps *maps = nullptr,
                         unsigned long long *mbar = nullptr) {
-  const int lane = threadIdx.x & 31;
-  const int nseg = A.nseg[d];
-  const int nchunk = A.nchunk;
-  const int chunk = (int)(wid % nchunk);
-  const int rest = wid / nchunk;
-  const int seg = (int)(rest % nseg);
-  const int outer = (int)(rest / nseg);
-  const int i = 32 * chunk + lane;
-  const bool act = !(i < A.lo[d][2] || i > A.hi[d][2]);
   unsigned mask = 0xffffffffu;
   bool leader = false;
+  int i, outer, seg, chunk = 0;
   if constexpr (TMA) {
+    // whole 32-cell row segments: one warp per i chunk, outer index and segment (blk: the warp)
+    chunk = blk % A.nchunk;
+    const int rest = blk / A.nchunk;
+    seg = rest % A.nseg[d];
+    outer = rest / A.nseg[d];
+    i = 32 * chunk + (threadIdx.x & 31);
+    const bool act = !(i < A.lo[d][2] || i > A.hi[d][2]);
     mask = __ballot_sync(0xffffffffu, act);
-    leader = act && (lane == __ffs(mask) - 1);
+    leader = act && ((threadIdx.x & 31) == __ffs(mask) - 1);
+    if (!act) return;
+  } else {
+    if (!yz_place(A, d, blk, i, outer, seg)) return;
   }
-  if (!act) return;
   const int sweep_lo = (d == 1) ? A.lo[1][1] : A.lo[2][0];
   const int sweep_hi = (d == 1) ? A.hi[1][1] : A.hi[2][0];
-  const int f0 = sweep_lo + A.seglen * seg;
-  const int f1 = min(f0 + A.seglen - 1, sweep_hi);
+  const int f0 = sweep_lo + A.slen[d] * seg;
+  const int f1 = min(f0 + A.slen[d] - 1, sweep_hi);
   const DirView<P> V = dir_view(A, d);
   const int st = V.st;
   int lc = (d == 1) ? A.g.idx32(A.lo[1][0] + outer, f0 - 1, i) : A.g.idx32(f0 - 1, A.lo[2][1] + outer, i);
@@ -701,24 +742,17 @@ CHQ_D void sweep_yz_ppm(const FluxArgs<P> &A, int d, int wid, P *park, P *win, c
 // asynchronous copy per quantity and cell, issued a whole cell ahead, instead of 2RE+1
 // cached loads whose lines a y/z march cannot keep in L1.
 template <int R, int S, bool CHAR, bool WIN, class P>
-CHQ_D void sweep_yz(const FluxArgs<P> &A, int d, int wid, P *park, P *win) {
+CHQ_D void sweep_yz(const FluxArgs<P> &A, int d, int blk, P *park, P *win) {
   if constexpr (R == R_PPM && !CHAR && WIN) {
-    sweep_yz_ppm<S, P>(A, d, wid, park, win);
+    sweep_yz_ppm<S, P>(A, d, blk, park, win);
     return;
   }
-  const int lane = threadIdx.x & 31;
-  const int nseg = A.nseg[d];
-  const int nchunk = A.nchunk;
-  const int chunk = (int)(wid % nchunk);
-  const int rest = wid / nchunk;
-  const int seg = (int)(rest % nseg);
-  const int outer = (int)(rest / nseg);
-  const int i = 32 * chunk + lane;
-  if (i < A.lo[d][2] || i > A.hi[d][2]) return;
+  int i, outer, seg;
+  if (!yz_place(A, d, blk, i, outer, seg)) return;
   const int sweep_lo = (d == 1) ? A.lo[1][1] : A.lo[2][0];
   const int sweep_hi = (d == 1) ? A.hi[1][1] : A.hi[2][0];
-  const int f0 = sweep_lo + A.seglen * seg;
-  const int f1 = min(f0 + A.seglen - 1, sweep_hi);
+  const int f0 = sweep_lo + A.slen[d] * seg;
+  const int f1 = min(f0 + A.slen[d] - 1, sweep_hi);
   const DirView<P> V = dir_view(A, d);
   // cell f0-1 first (its right state only), then cell f and face f for f = f0..f1; one copy
   // of the cell code in the loop keeps the kernel's instruction footprint small
@@ -811,7 +845,7 @@ template <int R, int S, bool CHAR, class P, int V = 0>
 __global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_kernel(const __grid_constant__ FluxArgs<P> A) {
   if (A.skip && *A.skip) return;
   const int wid = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 5);
-  if (wid < (int)A.nwarp[0]) {
+  if (wid < A.nxwarp) {
     if constexpr (R == R_PPM && !CHAR) sweep_x_ppm<S, P>(A, wid);
     else sweep_x<R, S, CHAR, P>(A, wid);
   }
@@ -823,15 +857,20 @@ __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<P>::v) flux_yz_ker
   P *park = reinterpret_cast<P *>(flux_dsm);
   P *win = park + 8 * kYzThreads;
   if (A.skip && *A.skip) return;
-  const int wid = (int)blockIdx.x * (kYzThreads / 32) + (int)(threadIdx.x >> 5);
-  const int nz = (int)A.nwarp[2], nyz = (int)(A.nwarp[2] + A.nwarp[1]);
-  if (wid < nz) sweep_yz<R, S, CHAR, true, P>(A, 2, wid, park, win);
-  else if (wid < nyz) sweep_yz<R, S, CHAR, true, P>(A, 1, wid - nz, park, win);
+  const int b = (int)blockIdx.x;
+  if (b < A.nblk[2]) sweep_yz<R, S, CHAR, true, P>(A, 2, b, park, win);
+  else if (b < A.nblk[2] + A.nblk[1]) sweep_yz<R, S, CHAR, true, P>(A, 1, b - A.nblk[2], park, win);
 }
 
 // The FP64 streaming-PPM y/z kernel with TMA staging (FluxArgs::yzvar = 1): dynamic shared
 // memory of flux_yz_kernel plus one mbarrier per warp; the tensor maps are kernel parameters.
 constexpr size_t flux_yz_tma_smem() { return flux_yz_smem<R_PPM, double>() + (kYzThreads / 32) * sizeof(unsigned long long); }
+
+// its warps of direction d
+template <class P> CHQ_HD int tma_warps(const FluxArgs<P> &A, int d) {
+  const int o = (d == 1) ? 0 : 1;   // the outer index: k for y sweeps, j for z sweeps
+  return A.nblk[d] ? A.nchunk * (A.hi[d][o] - A.lo[d][o] + 1) * A.nseg[d] : 0;
+}
 
 template <int S>
 __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<double>::v)
@@ -842,7 +881,7 @@ __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<double>::v)
   unsigned long long *mbar = reinterpret_cast<unsigned long long *>(flux_tma_dsm + flux_yz_smem<R_PPM, double>());
   if (A.skip && *A.skip) return;
   const int wid = (int)blockIdx.x * (kYzThreads / 32) + (int)(threadIdx.x >> 5);
-  const int nz = (int)A.nwarp[2], nyz = (int)(A.nwarp[2] + A.nwarp[1]);
+  const int nz = tma_warps(A, 2), nyz = nz + tma_warps(A, 1);
   if (wid < nz) sweep_yz_ppm<S, double, true>(A, 2, wid, park, win, &maps, mbar);
   else if (wid < nyz) sweep_yz_ppm<S, double, true>(A, 1, wid - nz, park, win, &maps, mbar);
 }
@@ -856,7 +895,7 @@ __global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_batched(
   const FluxArgs<P> &A = stage_args(args, j, sa);
   if (A.skip && *A.skip) return;
   const int wid = (int)(blockIdx.x - slots[j].off) * 4 + (int)(threadIdx.x >> 5);
-  if (wid < (int)A.nwarp[0]) {
+  if (wid < A.nxwarp) {
     if constexpr (R == R_PPM && !CHAR) sweep_x_ppm<S, P>(A, wid);
     else sweep_x<R, S, CHAR, P>(A, wid);
   }
@@ -874,10 +913,9 @@ __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<P>::v) flux_yz_bat
   const int j = batch_job(slots, n, blockIdx.x);
   const FluxArgs<P> &A = stage_args(args, j, flux_dsm + flux_yz_smem<R, P>());
   if (A.skip && *A.skip) return;
-  const int wid = (int)(blockIdx.x - slots[j].off) * (kYzThreads / 32) + (int)(threadIdx.x >> 5);
-  const int nz = (int)A.nwarp[2], nyz = (int)(A.nwarp[2] + A.nwarp[1]);
-  if (wid < nz) sweep_yz<R, S, CHAR, true, P>(A, 2, wid, park, win);
-  else if (wid < nyz) sweep_yz<R, S, CHAR, true, P>(A, 1, wid - nz, park, win);
+  const int b = (int)(blockIdx.x - slots[j].off);
+  if (b < A.nblk[2]) sweep_yz<R, S, CHAR, true, P>(A, 2, b, park, win);
+  else if (b < A.nblk[2] + A.nblk[1]) sweep_yz<R, S, CHAR, true, P>(A, 1, b - A.nblk[2], park, win);
 }
 
 }  // namespace chq

@@ -27,9 +27,8 @@ static cudaError_t allow_smem(K kern, size_t smem, bool *ready) {
 
 // y/z sweeps (shared marching window, dynamic shared memory) then the x-sweep, one stream
 template <int S, bool C>
-static cudaError_t go(const FluxArgs<CHQ_P> &a, unsigned, cudaStream_t s) {
-  constexpr int wpb = kYzThreads / 32;
-  const unsigned nyz = (unsigned)((a.nwarp[1] + a.nwarp[2] + wpb - 1) / wpb), nx = (unsigned)((a.nwarp[0] + 3) / 4);
+static cudaError_t go(const FluxArgs<CHQ_P> &a, cudaStream_t s) {
+  const unsigned nyz = (unsigned)(a.nblk[1] + a.nblk[2]), nx = (unsigned)((a.nxwarp + 3) / 4);
   bool yz_done = false;
   if constexpr (CHQ_R == R_PPM && !C && sizeof(CHQ_P) == 8) {
     // TMA staging of the streaming-PPM march (picked by the autotuner; FP64 only)
@@ -40,7 +39,8 @@ static cudaError_t go(const FluxArgs<CHQ_P> &a, unsigned, cudaStream_t s) {
       if (ea != cudaSuccess) return ea;
       YzMaps maps;
       std::memcpy(&maps, a.yzmaps, sizeof(maps));
-      flux_yz_tma_kernel<S><<<nyz, kYzThreads, smem, s>>>(a, maps);
+      constexpr int wpb = kYzThreads / 32;
+      flux_yz_tma_kernel<S><<<(tma_warps(a, 1) + tma_warps(a, 2) + wpb - 1) / wpb, kYzThreads, smem, s>>>(a, maps);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       yz_done = true;
@@ -63,14 +63,12 @@ static cudaError_t go(const FluxArgs<CHQ_P> &a, unsigned, cudaStream_t s) {
 }
 
 template <>
-cudaError_t launch_flux<CHQ_P, CHQ_R>(const FluxArgs<CHQ_P> &a, int rsolver, int charac, unsigned nblocks,
-                                       cudaStream_t s) {
-  if (nblocks == 0) return cudaSuccess;
+cudaError_t launch_flux<CHQ_P, CHQ_R>(const FluxArgs<CHQ_P> &a, int rsolver, int charac, cudaStream_t s) {
   const bool c = (charac != 0) && (CHQ_R != R_DC);
   switch (rsolver) {
-    case S_HLLE: return c ? go<S_HLLE, true>(a, nblocks, s) : go<S_HLLE, false>(a, nblocks, s);
-    case S_HLLD: return c ? go<S_HLLD, true>(a, nblocks, s) : go<S_HLLD, false>(a, nblocks, s);
-    case S_LHLLD: return c ? go<S_LHLLD, true>(a, nblocks, s) : go<S_LHLLD, false>(a, nblocks, s);
+    case S_HLLE: return c ? go<S_HLLE, true>(a, s) : go<S_HLLE, false>(a, s);
+    case S_HLLD: return c ? go<S_HLLD, true>(a, s) : go<S_HLLD, false>(a, s);
+    case S_LHLLD: return c ? go<S_LHLLD, true>(a, s) : go<S_LHLLD, false>(a, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -7,7 +7,7 @@
 namespace chq {
 
 template <class P, int R>
-cudaError_t launch_flux(const FluxArgs<P> &a, int rsolver, int charac, unsigned nblocks, cudaStream_t s);
+cudaError_t launch_flux(const FluxArgs<P> &a, int rsolver, int charac, cudaStream_t s);
 
 // x-sweep blocks and y/z-sweep blocks of many meshes, with one slot table each
 template <class P, int R>

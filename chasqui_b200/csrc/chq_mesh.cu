@@ -373,6 +373,48 @@ enum { PK_FLUX = 0, PK_CORNER = 1, PK_UPDATE = 2, PK_FLAG = 3, PK_REPAIR = 4, PK
        PK_CTL = 8, PK_DIFF = 9, PK_STS = 10 };
 
 // ---- fluxes --------------------------------------------------------------------------
+// columns and march segments of direction d (1, 2) at a march length: the fewest segments of
+// at most that many faces, of equal lengths but for the last
+struct YzShape {
+  int ncol, nseg, slen;
+};
+YzShape yz_shape(const chq_mesh *m, int d, int len) {
+  const int s = (d == 1) ? 1 : 0, o = 1 - s;   // the swept and the outer index of (k, j, i)
+  const int nf = m->hi[d][s] - m->lo[d][s] + 1;
+  YzShape y;
+  y.ncol = (m->hi[d][2] - m->lo[d][2] + 1) * (m->hi[d][o] - m->lo[d][o] + 1);
+  y.nseg = (nf + len - 1) / len;
+  y.slen = (nf + y.nseg - 1) / y.nseg;
+  y.nseg = (nf + y.slen - 1) / y.slen;
+  return y;
+}
+
+// Default march length. A thread reconstructs one cell more than the faces it solves (about
+// 0.6 of a face's work), and the launch runs in waves of the resident blocks: the length with
+// the least waves x (length + 0.6). Small meshes thus take one face a thread (OT 64^2: 22 us a
+// flux launch at length 4, the old rule's), large ones the longest march.
+int default_march(const chq_mesh *m) {
+  const double resident = 148.0 * (m->mixed ? 6 : 3);   // y/z blocks of the PPM kernels (FluxYzMinBlocks)
+  int best = 4;
+  double least = 1e300;
+  for (int L : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64}) {
+    double blocks = 0.0, len = 1.0;
+    for (int d = 1; d < 3; ++d) {
+      if (!m->active[d]) continue;
+      const YzShape y = yz_shape(m, d, L);
+      blocks += (double)((y.ncol + kYzThreads - 1) / kYzThreads) * y.nseg;
+      len = std::max(len, (double)y.slen);
+    }
+    const double waves = (blocks < 4.0 * resident) ? std::ceil(blocks / resident) : blocks / resident + 0.5;
+    const double cost = std::max(waves, 1.0) * (len + 0.6);
+    if (cost < 0.999 * least) {
+      least = cost;
+      best = L;
+    }
+  }
+  return best;
+}
+
 template <class P>
 FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask) {
   FluxArgs<P> a{};
@@ -392,35 +434,39 @@ FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask) {
   a.low_mach = m->cfg.low_mach;
   a.lhlld_phi = m->cfg.lhlld_phi;
   a.rgm1 = P(1) / P(m->eos.gm1);
-  a.seglen = m->seglen;
   a.xvar = m->xvar;
   a.yzvar = m->tma_ok ? m->yzvar : 0;
   a.yzmaps = m->tma_ok ? &m->tmaps : nullptr;
   a.err = &m->ctl->err;
   a.nchunk = (m->g.ni + 1 + 31) / 32;
-  // x: rows x segments of XFaces faces (29 for streaming PPM, else 31); y/z: i chunks x
-  // outer x segments
-  const int xf = (m->cfg.recon == R_PPM && !m->cfg.characteristic) ? XFaces<R_PPM, false>::v : XFaces<R_DC, false>::v;
-  a.nseg[0] = (m->hi[0][2] - m->lo[0][2] + 1 + xf - 1) / xf;
-  a.nwarp[0] = a.active[0] ? (long)(m->hi[0][0] - m->lo[0][0] + 1) * (m->hi[0][1] - m->lo[0][1] + 1) * a.nseg[0] : 0;
-  a.nseg[1] = (m->hi[1][1] - m->lo[1][1] + 1 + a.seglen - 1) / a.seglen;
-  a.nwarp[1] = a.active[1] ? (long)a.nchunk * (m->hi[1][0] - m->lo[1][0] + 1) * a.nseg[1] : 0;
-  a.nseg[2] = (m->hi[2][0] - m->lo[2][0] + 1 + a.seglen - 1) / a.seglen;
-  a.nwarp[2] = a.active[2] ? (long)a.nchunk * (m->hi[2][1] - m->lo[2][1] + 1) * a.nseg[2] : 0;
+  // x: the rows end to end, 32 - XFaces lanes of overlap between warps
+  const bool stream = (m->cfg.recon == R_PPM && !m->cfg.characteristic);
+  const int per = stream ? XFaces<R_PPM, false>::v : XFaces<R_DC, false>::v;
+  const int lead = stream ? XFaces<R_PPM, false>::lead : XFaces<R_DC, false>::lead;
+  a.nxent = m->hi[0][2] - m->lo[0][2] + 1 + lead;
+  a.nxrow = (m->hi[0][0] - m->lo[0][0] + 1) * (m->hi[0][1] - m->lo[0][1] + 1);
+  // the last place holds a cell after the last face (streaming) or that face's right cell
+  const long places = (long)a.nxent * a.nxrow;
+  a.nxwarp = a.active[0] ? (int)std::max(1L, (places - (32 - per) + per - 1) / per) : 0;
+  for (int d = 1; d < 3; ++d) {
+    const YzShape y = yz_shape(m, d, m->seglen);
+    a.slen[d] = y.slen;
+    a.nseg[d] = y.nseg;
+    a.ncol[d] = y.ncol;
+    a.nblk[d] = a.active[d] ? (y.ncol + kYzThreads - 1) / kYzThreads * y.nseg : 0;
+  }
   a.skip = nullptr;
   return a;
 }
 
 template <class P>
 cudaError_t launch_flux_any(const FluxArgs<P> &a, int recon, int rsolver, int charac, cudaStream_t s) {
-  const long warps = a.nwarp[0] + a.nwarp[1] + a.nwarp[2];
-  const unsigned nblocks = (unsigned)((warps + 3) / 4);
   switch (recon) {
-    case R_DC: return launch_flux<P, R_DC>(a, rsolver, charac, nblocks, s);
-    case R_PLM: return launch_flux<P, R_PLM>(a, rsolver, charac, nblocks, s);
-    case R_PPM: return launch_flux<P, R_PPM>(a, rsolver, charac, nblocks, s);
-    case R_PPMX: return launch_flux<P, R_PPMX>(a, rsolver, charac, nblocks, s);
-    case R_WENOZ: return launch_flux<P, R_WENOZ>(a, rsolver, charac, nblocks, s);
+    case R_DC: return launch_flux<P, R_DC>(a, rsolver, charac, s);
+    case R_PLM: return launch_flux<P, R_PLM>(a, rsolver, charac, s);
+    case R_PPM: return launch_flux<P, R_PPM>(a, rsolver, charac, s);
+    case R_PPMX: return launch_flux<P, R_PPMX>(a, rsolver, charac, s);
+    case R_WENOZ: return launch_flux<P, R_WENOZ>(a, rsolver, charac, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1457,11 +1503,11 @@ int batch_build(chq_batch *B) {
   size_t o_flux_s, o_corner_s, o_update_s, o_flag_s, o_repair_s, o_limit_s, o_bc_s[3], o_c2p_s;
   o_flux_s = slots_of(h, J, [](chq_mesh *m) {
     const FluxArgs<P> a = flux_args<P>(m, 0, 7u);
-    return linear(a.nwarp[0] * 32, 128);
+    return linear((long)a.nxwarp * 32, 128);
   }, B->k_flux.nblocks);
   const size_t o_flux_yz_s = slots_of(h, J, [](chq_mesh *m) {
     const FluxArgs<P> a = flux_args<P>(m, 0, 7u);
-    return linear((a.nwarp[1] + a.nwarp[2]) * 32, kYzThreads);
+    return linear((long)(a.nblk[1] + a.nblk[2]) * kYzThreads, kYzThreads);
   }, B->k_flux_yz.nblocks);
   o_corner_s = slots_of(h, J, [](chq_mesh *m) { return corner_grid(m); }, B->k_corner.nblocks);
   o_update_s = slots_of(h, J, [](chq_mesh *m) { return update_grid(m); }, B->k_update.nblocks);
@@ -2196,22 +2242,7 @@ int mesh_create_impl(const chq_config *cfg, int nslab, int rank, chq_mesh **out)
   m->active[0] = 1;
   m->active[1] = g.two_d;
   m->active[2] = g.three_d;
-  // default march length: the longest of 16, 8, 4 that still gives the y/z sweeps a full
-  // device of threads (148 SMs x 1024), so that small meshes are not one long serial march
-  // per thread (chq_autotune measures instead)
-  {
-    const long lanes = (long)((g.ni + 1 + 31) / 32) * 32;
-    m->seglen = 4;
-    for (int L : {16, 8}) {
-      long threads = 0;
-      if (g.two_d) threads += lanes * (m->hi[1][0] - m->lo[1][0] + 1) * ((m->hi[1][1] - m->lo[1][1] + 1 + L - 1) / L);
-      if (g.three_d) threads += lanes * (m->hi[2][1] - m->lo[2][1] + 1) * ((m->hi[2][0] - m->lo[2][0] + 1 + L - 1) / L);
-      if (threads >= 148L * 1024) {
-        m->seglen = L;
-        break;
-      }
-    }
-  }
+  m->seglen = default_march(m);
 
   // one slab: doubles (u0, u1: 6 each; 6 face fields), P fields (w 6, bcc 3, ecc 3,
   // fluxes 18, face EMFs 6, edge EMFs 3), the int flag array, control block and scratch

@@ -219,8 +219,8 @@ CHQ_API int chq_profile(chq_mesh *m, int enable);
  * Kokkos range policy) ---------------------------------------------------------------------
  * Two knobs of the face-flux launch, neither of which changes any result bit:
  *  - march length = faces each thread of the y/z sweeps carries its cell states across
- *    (CHQ_TUNE_LENGTHS). The default is the longest of 16, 8, 4 that keeps a full device of
- *    y/z threads busy (16 from about 128^3 up, 4 for small meshes);
+ *    (CHQ_TUNE_LENGTHS). The default balances the waves of resident blocks against the one
+ *    cell a thread computes beyond its faces (1 on small meshes, longer on large ones);
  *  - x-sweep variant = the register cap the x-sweep kernel is compiled for (0: 4 resident
  *    128-thread blocks per SM in FP64 / 8 in FP32; 1: 5 / 10, more resident warps, fewer
  *    registers). Default 0. The tuner varies it in the FP64 form only: there both builds
