@@ -331,7 +331,7 @@ template <class T> CHQ_D T flow_speed_q(const MState<T> &s, T bn) {
   const T root = sqrt_q(disc);
   const T h = T(0.5) * (a + (disc > RootFloor<T>::v ? root : T(0)));
   const T r = sqrt_q(h);
-  return (h > RootFloor<T>::v) ? r : T(0);
+  return (h <= RootFloor<T>::v) ? T(0) : r;   // (a NaN stays one)
 }
 
 // single-star transverse velocity and field of one side (star_side); dm = rho (S - u), sms = S - S_M
