@@ -144,9 +144,10 @@ template <class P> CHQ_D void diff_flux_body(const DiffArgs<P> &A, int bx) {
   }
 }
 
-template <class P> __global__ void __launch_bounds__(256) diff_flux_kernel(const DiffArgs<P> A) { diff_flux_body<P>(A, blockIdx.x); }
+template <class P> __global__ void __launch_bounds__(256) diff_flux_kernel(const DiffArgs<P> A) { pdl_begin(); diff_flux_body<P>(A, blockIdx.x); }
 
 template <class P> __global__ void __launch_bounds__(256) diff_flux_batched(const DiffArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   const int j = batch_job(slots, n, blockIdx.x);
   __shared__ __align__(16) unsigned char sa[sizeof(DiffArgs<P>)];
   const DiffArgs<P> &A = stage_args(args, j, sa);
@@ -180,10 +181,12 @@ template <class P> CHQ_D void resistive_emf_body(const ResEmfArgs<P> &A, int bx,
 }
 
 template <class P> __global__ void __launch_bounds__(256) resistive_emf_kernel(const ResEmfArgs<P> A) {
+  pdl_begin();
   resistive_emf_body<P>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 template <class P> __global__ void __launch_bounds__(256) resistive_emf_batched(const ResEmfArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   int bx, by, bz;
   const int j = batch_job(slots, n, blockIdx.x);
   batch_block(slots[j], blockIdx.x, bx, by, bz);
@@ -214,10 +217,12 @@ template <class P> CHQ_D void rho_min_body(const RhoMinArgs<P> &A, int bx, int b
 }
 
 template <class P> __global__ void __launch_bounds__(256) rho_min_kernel(const RhoMinArgs<P> A) {
+  pdl_begin();
   rho_min_body<P>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 template <class P> __global__ void __launch_bounds__(256) rho_min_batched(const RhoMinArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   int bx, by, bz;
   const int j = batch_job(slots, n, blockIdx.x);
   batch_block(slots[j], blockIdx.x, bx, by, bz);
@@ -274,6 +279,7 @@ template <class P> CHQ_D void sts_div_body(const StsDivArgs<P> &A, int bx, int b
 }
 
 template <class P> __global__ void __launch_bounds__(256) sts_div_kernel(const StsDivArgs<P> A) {
+  pdl_begin();
   sts_div_body<P>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -310,6 +316,7 @@ CHQ_D void sts_combine_body(const StsCombArgs &A, const double *cf, int bx, int 
 }
 
 __global__ void __launch_bounds__(256) sts_combine_kernel(const StsCombArgs A) {
+  pdl_begin();
   const double cf[5] = {A.a, A.b, A.c, A.d, A.e};
   sts_combine_body(A, cf, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -318,11 +325,13 @@ __global__ void __launch_bounds__(256) sts_combine_kernel(const StsCombArgs A) {
 // Every member advances its own stage count s_m; at stage j the members with j > s_m (or a
 // finished clock) skip: skip[m] is rewritten before each stage.
 __global__ void sts_skip_kernel(int *skip, const int *nst, int n, int j) {
+  pdl_begin();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < n) skip[m] = (j > nst[m]) ? 1 : 0;
 }
 
 template <class P> __global__ void __launch_bounds__(256) sts_div_batched(const StsDivArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   int bx, by, bz;
   const int j = batch_job(slots, n, blockIdx.x);
   batch_block(slots[j], blockIdx.x, bx, by, bz);
@@ -334,6 +343,7 @@ template <class P> __global__ void __launch_bounds__(256) sts_div_batched(const 
 // coef: this stage's five coefficients of every member (member m at coef[5 m])
 __global__ void __launch_bounds__(256) sts_combine_batched(const StsCombArgs *args, const BatchSlot *slots, int n,
                                                            const double *coef) {
+  pdl_begin();
   int bx, by, bz;
   const int j = batch_job(slots, n, blockIdx.x);
   batch_block(slots[j], blockIdx.x, bx, by, bz);
@@ -354,6 +364,7 @@ struct SpanArgs {
 
 // the same copies and zero fills for one mesh (all blocks of the launch)
 __global__ void __launch_bounds__(256) span_kernel(const SpanArgs A) {
+  pdl_begin();
   for (int q = 0; q < A.nspan; ++q) {
     unsigned long long *d = A.dst[q];
     const unsigned long long *src = A.src[q];
@@ -363,6 +374,7 @@ __global__ void __launch_bounds__(256) span_kernel(const SpanArgs A) {
 }
 
 __global__ void __launch_bounds__(256) span_batched(const SpanArgs *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   const int j = batch_job(slots, n, blockIdx.x);
   __shared__ __align__(16) unsigned char sa[sizeof(SpanArgs)];
   const SpanArgs &A = stage_args(args, j, sa);

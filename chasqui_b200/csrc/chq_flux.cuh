@@ -843,16 +843,21 @@ template <int R, class P> __host__ __device__ constexpr size_t flux_yz_smem() {
 
 template <int R, int S, bool CHAR, class P, int V = 0>
 __global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_kernel(const __grid_constant__ FluxArgs<P> A) {
-  if (A.skip && *A.skip) return;
+  // The x sweep reads and writes nothing of the y/z launch before it, whose blocks have all
+  // passed their own wait when this one starts: it runs beside the y/z launch's last wave and
+  // waits for it at the end, so that it completes last. Alone it waits first.
+  if (A.nblk[1] + A.nblk[2] == 0) pdl_wait();
   const int wid = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 5);
-  if (wid < A.nxwarp) {
+  if (!(A.skip && *A.skip) && wid < A.nxwarp) {
     if constexpr (R == R_PPM && !CHAR) sweep_x_ppm<S, P>(A, wid);
     else sweep_x<R, S, CHAR, P>(A, wid);
   }
+  pdl_wait();
 }
 
 template <int R, int S, bool CHAR, class P>
 __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<P>::v) flux_yz_kernel(const __grid_constant__ FluxArgs<P> A) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char flux_dsm[];
   P *park = reinterpret_cast<P *>(flux_dsm);
   P *win = park + 8 * kYzThreads;
@@ -875,6 +880,7 @@ template <class P> CHQ_HD int tma_warps(const FluxArgs<P> &A, int d) {
 template <int S>
 __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<double>::v)
     flux_yz_tma_kernel(const __grid_constant__ FluxArgs<double> A, const __grid_constant__ YzMaps maps) {
+  pdl_begin();
   extern __shared__ __align__(128) unsigned char flux_tma_dsm[];
   double *park = reinterpret_cast<double *>(flux_tma_dsm);
   double *win = park + 8 * kYzThreads;
@@ -889,16 +895,17 @@ __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<double>::v)
 // batched forms: the blocks of many meshes in one launch per sweep kind (chq_batch); each
 // block copies its mesh's arguments to shared memory first
 template <int R, int S, bool CHAR, class P, int V = 0>
-__global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_batched(const FluxArgs<P> *args, const BatchSlot *slots, int n) {
+__global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_batched(const FluxArgs<P> *args, const BatchSlot *slots, int n, int alone) {
+  if (alone) pdl_wait();   // as in flux_x_kernel: no y/z launch before this one
   __shared__ __align__(16) unsigned char sa[sizeof(FluxArgs<P>)];
   const int j = batch_job(slots, n, blockIdx.x);
   const FluxArgs<P> &A = stage_args(args, j, sa);
-  if (A.skip && *A.skip) return;
   const int wid = (int)(blockIdx.x - slots[j].off) * 4 + (int)(threadIdx.x >> 5);
-  if (wid < A.nxwarp) {
+  if (!(A.skip && *A.skip) && wid < A.nxwarp) {
     if constexpr (R == R_PPM && !CHAR) sweep_x_ppm<S, P>(A, wid);
     else sweep_x<R, S, CHAR, P>(A, wid);
   }
+  pdl_wait();
 }
 
 template <int R, class P> __host__ __device__ constexpr size_t flux_yz_batched_smem() {
@@ -907,6 +914,7 @@ template <int R, class P> __host__ __device__ constexpr size_t flux_yz_batched_s
 
 template <int R, int S, bool CHAR, class P>
 __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<P>::v) flux_yz_batched(const FluxArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char flux_dsm[];
   P *park = reinterpret_cast<P *>(flux_dsm);
   P *win = park + 8 * kYzThreads;

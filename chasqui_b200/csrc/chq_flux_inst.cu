@@ -40,7 +40,7 @@ static cudaError_t go(const FluxArgs<CHQ_P> &a, cudaStream_t s) {
       YzMaps maps;
       std::memcpy(&maps, a.yzmaps, sizeof(maps));
       constexpr int wpb = kYzThreads / 32;
-      flux_yz_tma_kernel<S><<<(tma_warps(a, 1) + tma_warps(a, 2) + wpb - 1) / wpb, kYzThreads, smem, s>>>(a, maps);
+      pdl(flux_yz_tma_kernel<S>, (tma_warps(a, 1) + tma_warps(a, 2) + wpb - 1) / wpb, kYzThreads, smem, s, a, maps);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       yz_done = true;
@@ -51,13 +51,13 @@ static cudaError_t go(const FluxArgs<CHQ_P> &a, cudaStream_t s) {
     static bool ready[64] = {};
     const cudaError_t ea = allow_smem(flux_yz_kernel<CHQ_R, S, C, CHQ_P>, smem, ready);
     if (ea != cudaSuccess) return ea;
-    flux_yz_kernel<CHQ_R, S, C, CHQ_P><<<nyz, kYzThreads, smem, s>>>(a);
+    pdl(flux_yz_kernel<CHQ_R, S, C, CHQ_P>, nyz, kYzThreads, smem, s, a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   if (nx) {
-    if (a.xvar) flux_x_kernel<CHQ_R, S, C, CHQ_P, 1><<<nx, 128, 0, s>>>(a);
-    else flux_x_kernel<CHQ_R, S, C, CHQ_P, 0><<<nx, 128, 0, s>>>(a);
+    if (a.xvar) pdl(flux_x_kernel<CHQ_R, S, C, CHQ_P, 1>, nx, 128, 0, s, a);
+    else pdl(flux_x_kernel<CHQ_R, S, C, CHQ_P, 0>, nx, 128, 0, s, a);
   }
   return cudaGetLastError();
 }
@@ -81,13 +81,13 @@ static cudaError_t gob(const FluxArgs<CHQ_P> *a, const BatchSlot *sx, const Batc
     static bool ready[64] = {};
     const cudaError_t e = allow_smem(flux_yz_batched<CHQ_R, S, C, CHQ_P>, smem, ready);
     if (e != cudaSuccess) return e;
-    flux_yz_batched<CHQ_R, S, C, CHQ_P><<<nbyz, kYzThreads, smem, s>>>(a, syz, n);
+    pdl(flux_yz_batched<CHQ_R, S, C, CHQ_P>, nbyz, kYzThreads, smem, s, a, syz, n);
     const cudaError_t e2 = cudaGetLastError();
     if (e2 != cudaSuccess) return e2;
   }
   if (nbx) {
-    if (xvar) flux_x_batched<CHQ_R, S, C, CHQ_P, 1><<<nbx, 128, 0, s>>>(a, sx, n);
-    else flux_x_batched<CHQ_R, S, C, CHQ_P, 0><<<nbx, 128, 0, s>>>(a, sx, n);
+    if (xvar) pdl(flux_x_batched<CHQ_R, S, C, CHQ_P, 1>, nbx, 128, 0, s, a, sx, n, nbyz == 0);
+    else pdl(flux_x_batched<CHQ_R, S, C, CHQ_P, 0>, nbx, 128, 0, s, a, sx, n, nbyz == 0);
   }
   return cudaGetLastError();
 }

@@ -69,13 +69,15 @@ CHQ_D void ctl_end(StepCtl *c) {
   c->min_dt = __longlong_as_double((long long)c->mdt_bits);
   if (c->diff_on && !c->sts) c->min_dt = fmin(c->min_dt, parabolic_dt(c));
 }
-__global__ void ctl_begin_kernel(StepCtl *c, int) { ctl_begin(c); }
-__global__ void ctl_end_kernel(StepCtl *c) { ctl_end(c); }
+__global__ void ctl_begin_kernel(StepCtl *c, int) { pdl_begin(); ctl_begin(c); }
+__global__ void ctl_end_kernel(StepCtl *c) { pdl_begin(); ctl_end(c); }
 __global__ void ctl_begin_batched(StepCtl *const *c, int n) {
+  pdl_begin();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < n) ctl_begin(c[j]);
 }
 __global__ void ctl_end_batched(StepCtl *const *c, int n) {
+  pdl_begin();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < n) ctl_end(c[j]);
 }
@@ -522,7 +524,7 @@ int do_corner(chq_mesh *m, const int *done, const int *need, cudaStream_t s) {
   const EmfArgs<P> a = corner_args<P>(m, done, need);
   const Launch3 L = corner_grid(m);
   m->nlaunch += 1;
-  corner_emf_kernel<P><<<L.grid, L.block, 0, s>>>(a);
+  pdl(corner_emf_kernel<P>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -537,7 +539,7 @@ int do_corner_rerun(chq_mesh *m, const int *done, const int *need, cudaStream_t 
   const Geom &g = m->g;
   const long pts = (long)(g.ie + 2 - g.is) * (g.je + 2 - g.js) * (g.three_d ? g.ke + 2 - g.ks : 1);
   m->nlaunch += 1;
-  corner_rerun_kernel<P><<<repair_grid(pts, kRepairBlocks).grid, 256, 0, s>>>(a);
+  pdl(corner_rerun_kernel<P>, repair_grid(pts, kRepairBlocks).grid, 256, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -576,12 +578,12 @@ Launch3 update_grid(const chq_mesh *m) {
 
 template <class P>
 int do_update(chq_mesh *m, int out, double g0, double g1, double bdt, const double *bdt_dev, const int *done,
-              const int *need, cudaStream_t s) {
-  const UpdateArgs<P> a = update_args<P>(m, out, g0, g1, bdt, bdt_dev, done, need);
+              cudaStream_t s) {
+  const UpdateArgs<P> a = update_args<P>(m, out, g0, g1, bdt, bdt_dev, done, nullptr);
   const Launch3 L = update_grid(m);
   m->nlaunch += 1;
-  if (a.grav.on) update_kernel<P, true><<<L.grid, L.block, 0, s>>>(a);
-  else update_kernel<P, false><<<L.grid, L.block, 0, s>>>(a);
+  if (a.grav.on) pdl(update_kernel<P, true>, L.grid, L.block, 0, s, a);
+  else pdl(update_kernel<P, false>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -592,23 +594,24 @@ int do_update(chq_mesh *m, int out, double g0, double g1, double bdt, const doub
 template <class P>
 int do_update_rerun(chq_mesh *m, int out, double g0, double g1, double bdt, const double *bdt_dev, const int *done,
                     const int *need, cudaStream_t s) {
-  if (!(g1 == 0.0 && out == 1) || m->bad_cap <= 0) return do_update<P>(m, out, g0, g1, bdt, bdt_dev, done, need, s);
   UpdateArgs<P> a = update_args<P>(m, out, g0, g1, bdt, bdt_dev, done, need);
-  a.list = m->bad_list;
-  a.cap = m->bad_cap;
   const Geom &g = m->g;
-  const int per = 3 * (g.two_d ? 3 : 1) * (g.three_d ? 3 : 1);
-  const dim3 grid = repair_grid((long)per * m->bad_cap, kRepairBlocks).grid;
-  m->nlaunch += 2;
-  if (a.grav.on) update_rerun_listed_kernel<P, true><<<grid, 256, 0, s>>>(a);
-  else update_rerun_listed_kernel<P, false><<<grid, 256, 0, s>>>(a);
-  CHQ_CUDA(cudaGetLastError());
-  // list overflow (count above the capacity): the whole update, as in the other stages
-  a.need_min = m->bad_cap;
+  if (g1 == 0.0 && out == 1 && m->bad_cap > 0) {
+    a.list = m->bad_list;
+    a.cap = m->bad_cap;
+    const int per = 3 * (g.two_d ? 3 : 1) * (g.three_d ? 3 : 1);
+    const long cells = std::min((long)m->bad_cap, (long)g.nx1 * g.nx2 * g.nx3);
+    const dim3 grid = repair_grid(per * cells, kRepairBlocks).grid;
+    m->nlaunch += 1;
+    if (a.grav.on) CHQ_CUDA(pdl(update_rerun_listed_kernel<P, true>, grid, 256, 0, s, a));
+    else CHQ_CUDA(pdl(update_rerun_listed_kernel<P, false>, grid, 256, 0, s, a));
+    a.need_min = m->bad_cap;   // list overflow (count above the capacity): the whole update
+  }
   const Launch3 L = update_grid(m);
-  if (a.grav.on) update_kernel<P, true><<<L.grid, L.block, 0, s>>>(a);
-  else update_kernel<P, false><<<L.grid, L.block, 0, s>>>(a);
-  CHQ_CUDA(cudaGetLastError());
+  const unsigned blocks = (unsigned)std::min((long)L.grid.x * L.grid.y * L.grid.z, kRepairBlocks);
+  m->nlaunch += 1;
+  if (a.grav.on) CHQ_CUDA(pdl(update_rerun_kernel<P, true>, blocks, dim3(32, 8), 0, s, a));
+  else CHQ_CUDA(pdl(update_rerun_kernel<P, false>, blocks, dim3(32, 8), 0, s, a));
   return CHQ_OK;
 }
 
@@ -636,7 +639,7 @@ int do_flag(chq_mesh *m, int buf, int *nbad_dev, const int *done, cudaStream_t s
   const FlagArgs a = flag_args(m, buf, nbad_dev, done);
   const Launch3 L = flag_grid(m);
   m->nlaunch += 1;
-  fofc_flag_kernel<<<L.grid, L.block, 0, s>>>(a);
+  pdl(fofc_flag_kernel, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -681,7 +684,7 @@ int do_repair(chq_mesh *m, int cur, unsigned dirmask, const int *done, const int
   const RepairArgs<P> a = repair_args<P>(m, cur, dirmask, done, need, tot);
   if (tot == 0) return CHQ_OK;
   m->nlaunch += 1;
-  fofc_repair_kernel<P><<<repair_grid(tot, kRepairBlocks).grid, 256, 0, s>>>(a);
+  pdl(fofc_repair_kernel<P>, repair_grid(tot, kRepairBlocks).grid, 256, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -730,58 +733,36 @@ int do_limit(chq_mesh *m, unsigned dirmask, double bdt, const double *bdt_dev, l
   const LimitArgs<P> a = limit_args<P>(m, dirmask, bdt, bdt_dev, count_dev, done, tot);
   if (tot == 0) return CHQ_OK;
   m->nlaunch += 1;
-  limit_kernel<P><<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(a);
+  pdl(limit_kernel<P>, (unsigned)((tot + 255) / 256), 256, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
 
-BcArgs bc_args(chq_mesh *m, int buf, const int *done, int dir) {
+BcArgs bc_args_ptr(chq_mesh *m, double *u, double *b1, double *b2, double *b3, const int *done) {
   BcArgs a{};
   a.g = m->g;
-  a.u = m->u[buf];
-  a.b1 = m->bf[buf][0]; a.b2 = m->bf[buf][1]; a.b3 = m->bf[buf][2];
-  a.done = done;
-  a.bc = (dir == 0) ? m->cfg.bc1 : (dir == 1) ? m->cfg.bc2 : m->cfg.bc3;
-  a.zside = 3;
-  return a;
-}
-
-// threads of the ghost-fill launch of one direction (0 when the direction is inactive)
-long bc_threads(const chq_mesh *m, int dir) {
-  const Geom &g = m->g;
-  if (dir == 0) return (long)(g.nk + 1) * (g.nj + 1) * g.ng;
-  if (dir == 1) return g.two_d ? (long)(g.nk + 1) * g.ng * (g.ni + 1) : 0;
-  return g.three_d ? (long)g.ng * (g.nj + 1) * (g.ni + 1) : 0;
-}
-
-int do_bc_ptr(chq_mesh *m, double *u, double *b1, double *b2, double *b3, const int *done, cudaStream_t s) {
-  const Geom &g = m->g;
-  BcArgs a{};
-  a.g = g;
   a.u = u;
   a.b1 = b1; a.b2 = b2; a.b3 = b3;
   a.done = done;
-  a.bc = m->cfg.bc1;
-  long n = (long)(g.nk + 1) * (g.nj + 1) * g.ng;
-  m->nlaunch += 1;
-  bc_kernel<0><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
-  CHQ_CUDA(cudaGetLastError());
-  if (g.two_d) {
-    a.bc = m->cfg.bc2;
-    n = (long)(g.nk + 1) * g.ng * (g.ni + 1);
-    m->nlaunch += 1;
-    bc_kernel<1><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
-    CHQ_CUDA(cudaGetLastError());
-  }
+  a.bc[0] = m->cfg.bc1; a.bc[1] = m->cfg.bc2; a.bc[2] = m->cfg.bc3;
   // a z slab's peer sides receive halos from the neighbouring slabs instead (chq_slab_unpack)
   a.zside = (m->zpeer[0] ? 0 : 1) | (m->zpeer[1] ? 0 : 2);
-  if (g.three_d && a.zside) {
-    a.bc = m->cfg.bc3;
-    n = (long)g.ng * (g.nj + 1) * (g.ni + 1);
-    m->nlaunch += 1;
-    bc_kernel<2><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
-    CHQ_CUDA(cudaGetLastError());
-  }
+  return a;
+}
+
+BcArgs bc_args(chq_mesh *m, int buf, const int *done) {
+  return bc_args_ptr(m, m->u[buf], m->bf[buf][0], m->bf[buf][1], m->bf[buf][2], done);
+}
+
+// threads of the ghost-fill launch
+long bc_threads(const chq_mesh *m) {
+  const BcShape b = bc_shape(m->g);
+  return b.nz + b.ny + b.nx;
+}
+
+int do_bc_ptr(chq_mesh *m, double *u, double *b1, double *b2, double *b3, const int *done, cudaStream_t s) {
+  m->nlaunch += 1;
+  CHQ_CUDA(pdl(bc_kernel, (unsigned)((bc_threads(m) + 255) / 256), 256, 0, s, bc_args_ptr(m, u, b1, b2, b3, done)));
   return CHQ_OK;
 }
 
@@ -820,7 +801,7 @@ template <class P>
 int launch_c2p(chq_mesh *m, const C2pArgs<P> &a, cudaStream_t s) {
   const Launch3 L = c2p_grid(m);
   m->nlaunch += 1;
-  c2p_kernel<P><<<L.grid, L.block, 0, s>>>(a);
+  pdl(c2p_kernel<P>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -840,7 +821,7 @@ int do_c2p_end(chq_mesh *m, const int *done, cudaStream_t s) {
   a.hst = m->hrec;
   const Launch3 L = c2p_grid(m);
   m->nlaunch += 1;
-  c2p_kernel<P, true><<<L.grid, L.block, 0, s>>>(a);
+  pdl(c2p_kernel<P, true>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -892,7 +873,7 @@ int do_diff(chq_mesh *m, const double *b1, const double *b2, const double *b3, c
   const DiffArgs<P> a = diff_args<P>(m, b1, b2, b3, done, tot);
   if (tot == 0) return CHQ_OK;
   m->nlaunch += 1;
-  diff_flux_kernel<P><<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(a);
+  pdl(diff_flux_kernel<P>, (unsigned)((tot + 255) / 256), 256, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -929,7 +910,7 @@ int do_res_emf(chq_mesh *m, const double *b1, const double *b2, const double *b3
   if (!(m->cfg.eta > 0.0)) return CHQ_OK;
   const ResEmfArgs<P> a = res_emf_args<P>(m, b1, b2, b3, done, need);
   m->nlaunch += 1;
-  resistive_emf_kernel<P><<<res_emf_grid(m).grid, dim3(32, 8), 0, s>>>(a);
+  pdl(resistive_emf_kernel<P>, res_emf_grid(m).grid, dim3(32, 8), 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -964,7 +945,7 @@ int do_cooling(chq_mesh *m, const int *done, cudaStream_t s) {
   a.done = done;
   const dim3 grid((unsigned)((g.nx1 + 31) / 32), (unsigned)((g.je - g.js + 1 + 7) / 8), (unsigned)(g.ke - g.ks + 1));
   m->nlaunch += 1;
-  cooling_kernel<P><<<grid, dim3(32, 8), 0, s>>>(a);
+  pdl(cooling_kernel<P>, grid, dim3(32, 8), 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -975,7 +956,7 @@ int do_rho_min(chq_mesh *m, const int *done, cudaStream_t s) {
   const Geom &g = m->g;
   const dim3 grid((unsigned)((g.nx1 + 31) / 32), (unsigned)((g.je - g.js + 1 + 7) / 8), (unsigned)(g.ke - g.ks + 1));
   m->nlaunch += 1;
-  rho_min_kernel<P><<<grid, dim3(32, 8), 0, s>>>(rho_min_args<P>(m, done));
+  pdl(rho_min_kernel<P>, grid, dim3(32, 8), 0, s, rho_min_args<P>(m, done));
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -994,7 +975,7 @@ int do_repair_d(chq_mesh *m, int cur, bool with_diff, const int *done, const int
     a.diff = diff_args<P>(m, m->bf[cur][0], m->bf[cur][1], m->bf[cur][2], done, nd);
   }
   m->nlaunch += 1;
-  fofc_repair_kernel<P><<<repair_grid(tot, kRepairBlocks).grid, 256, 0, s>>>(a);
+  pdl(fofc_repair_kernel<P>, repair_grid(tot, kRepairBlocks).grid, 256, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -1031,7 +1012,7 @@ int run_stage_a(chq_mesh *m, int cur, int out, double g0, double g1, double bdt,
   }
   {
     Prof p(m, PK_UPDATE, s);
-    if ((rc = DISPATCH_P(m, do_update)(m, out, g0, g1, bdt, bdt_dev, done, nullptr, s))) return rc;
+    if ((rc = DISPATCH_P(m, do_update)(m, out, g0, g1, bdt, bdt_dev, done, s))) return rc;
   }
   if (m->cfg.fofc) {
     Prof p(m, PK_FLAG, s);
@@ -1092,7 +1073,7 @@ int launch_spans(chq_mesh *m, const SpanArgs &a, cudaStream_t s) {
   for (int q = 0; q < a.nspan; ++q) words = std::max(words, a.words[q]);
   const unsigned blocks = (unsigned)std::max(1L, std::min(1184L, (words + 1023) / 1024));
   m->nlaunch += 1;
-  span_kernel<<<blocks, 256, 0, s>>>(a);
+  pdl(span_kernel, blocks, 256, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -1123,7 +1104,7 @@ int sts_operator(chq_mesh *m, double *const b[3], double *mu, double *const mb[3
   a.idx1 = 1.0 / g.dx1; a.idx2 = 1.0 / g.dx2; a.idx3 = 1.0 / g.dx3;
   const Launch3 L = update_grid(m);
   m->nlaunch += 1;
-  sts_div_kernel<P><<<L.grid, L.block, 0, s>>>(a);
+  pdl(sts_div_kernel<P>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -1141,7 +1122,7 @@ int sts_combine(chq_mesh *m, const StsState &out, double a, const StsState &x, d
   }
   const Launch3 L = update_grid(m);
   m->nlaunch += 1;
-  sts_combine_kernel<<<L.grid, L.block, 0, s>>>(A);
+  pdl(sts_combine_kernel, L.grid, L.block, 0, s, A);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -1433,7 +1414,7 @@ struct chq_batch {
     BatchSlot *slots = nullptr;
     long nblocks = 0;
   };
-  Kind k_flux, k_flux_yz, k_corner, k_update, k_flag, k_repair, k_limit, k_bc[3], k_c2p;
+  Kind k_flux, k_flux_yz, k_corner, k_update, k_flag, k_repair, k_limit, k_bc, k_c2p;
   // source terms and diffusion (every member or none): with explicit diffusion (diff) the
   // stage adds the diffusive fluxes after K1 and eta J after the corner EMFs; gravity runs in
   // the update epilogue; cooling is split after the step
@@ -1444,14 +1425,14 @@ struct chq_batch {
   // built once; stage counts, coefficients and the final copies are uploaded every cycle
   Kind k_span;
   void *a_sts_c2p[4] = {}, *a_sts_diff[4] = {}, *a_sts_res[4] = {}, *a_sts_div[2] = {}, *a_sts_comb[5] = {},
-       *a_sts_bc[4][3] = {}, *a_sts_zero = nullptr, *a_sts_copy0 = nullptr;
+       *a_sts_bc[4] = {}, *a_sts_zero = nullptr, *a_sts_copy0 = nullptr;
   int *sts_skip = nullptr;   // per member: skip the current RKL2 stage
   char *sts_dyn = nullptr;   // per cycle: stage counts | coefficients | final copies
   size_t sts_dyn_bytes = 0;
   void *a_diff[4] = {}, *a_res[4] = {}, *a_res_need[4] = {};
-  void *a_rho = nullptr, *a_cool = nullptr, *a_c2p_split[2] = {}, *a_bc0[3] = {};
+  void *a_rho = nullptr, *a_cool = nullptr, *a_c2p_split[2] = {}, *a_bc0 = nullptr;
   void *a_flux[4] = {}, *a_update[4] = {}, *a_update_need[4] = {}, *a_repair[4] = {}, *a_limit[4] = {},
-       *a_c2p[4] = {}, *a_flag[4] = {}, *a_bc[4][3] = {};
+       *a_c2p[4] = {}, *a_flag[4] = {}, *a_bc[4] = {};
   void *a_corner = nullptr, *a_corner_need = nullptr;
   StepCtl **ctls = nullptr;
   double *status = nullptr;
@@ -1500,7 +1481,7 @@ int batch_build(chq_batch *B) {
   HostTable h;
   const std::vector<chq_mesh *> &J = B->jobs;
   const int n = (int)J.size();
-  size_t o_flux_s, o_corner_s, o_update_s, o_flag_s, o_repair_s, o_limit_s, o_bc_s[3], o_c2p_s;
+  size_t o_flux_s, o_corner_s, o_update_s, o_flag_s, o_repair_s, o_limit_s, o_bc_s, o_c2p_s;
   o_flux_s = slots_of(h, J, [](chq_mesh *m) {
     const FluxArgs<P> a = flux_args<P>(m, 0, 7u);
     return linear((long)a.nxwarp * 32, 128);
@@ -1522,8 +1503,7 @@ int batch_build(chq_batch *B) {
     limit_args<P>(m, 7u, 0.0, nullptr, nullptr, nullptr, tot);
     return linear(tot, 256);
   }, B->k_limit.nblocks);
-  for (int d = 0; d < 3; ++d)
-    o_bc_s[d] = slots_of(h, J, [d](chq_mesh *m) { return linear(bc_threads(m, d), 256); }, B->k_bc[d].nblocks);
+  o_bc_s = slots_of(h, J, [](chq_mesh *m) { return linear(bc_threads(m), 256); }, B->k_bc.nblocks);
   o_c2p_s = slots_of(h, J, [](chq_mesh *m) { return c2p_grid(m); }, B->k_c2p.nblocks);
   const size_t o_diff_s = slots_of(h, J, [](chq_mesh *m) {
     long tot = 0;
@@ -1552,13 +1532,13 @@ int batch_build(chq_batch *B) {
     ctls[j] = m->ctl;
   }
   const size_t o_corner = push_vec(h, corner), o_corner_need = push_vec(h, corner_need), o_ctls = push_vec(h, ctls);
-  size_t o_flux[4], o_update[4], o_update_need[4], o_flag[4], o_repair[4], o_limit[4], o_bc[4][3], o_c2p[4];
+  size_t o_flux[4], o_update[4], o_update_need[4], o_flag[4], o_repair[4], o_limit[4], o_bc[4], o_c2p[4];
   size_t o_diff[4] = {}, o_res[4] = {}, o_res_need[4] = {};
   // the cooling split: con2prim of u0 without and with the dt, cooling, boundaries of u0
   std::vector<RhoMinArgs<P>> rho(n);
   std::vector<CoolArgs<P>> cool(n);
   std::vector<C2pArgs<P>> split0(n), split1(n);
-  std::vector<BcArgs> bc0[3] = {std::vector<BcArgs>(n), std::vector<BcArgs>(n), std::vector<BcArgs>(n)};
+  std::vector<BcArgs> bc0(n);
   for (int j = 0; j < n; ++j) {
     chq_mesh *m = J[j];
     StepCtl *c = m->ctl;
@@ -1566,12 +1546,11 @@ int batch_build(chq_batch *B) {
     cool[j] = cool_args<P>(m, &c->done);
     split0[j] = c2p_args<P>(m, 0, 0, &c->mdt_bits, c, &c->done);
     split1[j] = c2p_args<P>(m, 0, 1, &c->mdt_bits, c, &c->done);
-    for (int d = 0; d < 3; ++d) bc0[d][j] = bc_args(m, 0, &c->done, d);
+    bc0[j] = bc_args(m, 0, &c->done);
   }
   const size_t o_rho = push_vec(h, rho), o_cool = push_vec(h, cool), o_split0 = push_vec(h, split0),
                o_split1 = push_vec(h, split1);
-  size_t o_bc0[3];
-  for (int d = 0; d < 3; ++d) o_bc0[d] = push_vec(h, bc0[d]);
+  const size_t o_bc0 = push_vec(h, bc0);
   for (int st = 1; st <= B->nstage; ++st) {
     double g0, g1, beta;
     int cur, out;
@@ -1582,7 +1561,7 @@ int batch_build(chq_batch *B) {
     std::vector<FlagArgs> fl(n);
     std::vector<RepairArgs<P>> ra(n);
     std::vector<LimitArgs<P>> la(n);
-    std::vector<BcArgs> bc[3] = {std::vector<BcArgs>(n), std::vector<BcArgs>(n), std::vector<BcArgs>(n)};
+    std::vector<BcArgs> bc(n);
     std::vector<C2pArgs<P>> ca(n);
     std::vector<DiffArgs<P>> da(n);
     std::vector<ResEmfArgs<P>> ea(n), ean(n);
@@ -1606,7 +1585,7 @@ int batch_build(chq_batch *B) {
         ra[j].diff = da[j];
       }
       la[j] = limit_args<P>(m, 7u, 0.0, &c->beta_dt[st - 1], &c->limiter_count, &c->done, tot);
-      for (int d = 0; d < 3; ++d) bc[d][j] = bc_args(m, out, &c->done, d);
+      bc[j] = bc_args(m, out, &c->done);
       const bool split = m->cfg.cooling || (m->diff && m->cfg.sts);
       ca[j] = c2p_args<P>(m, out, (last && !split) ? 1 : 0, &c->mdt_bits, c, &c->done);
     }
@@ -1619,13 +1598,13 @@ int batch_build(chq_batch *B) {
     o_flag[st - 1] = push_vec(h, fl);
     o_repair[st - 1] = push_vec(h, ra);
     o_limit[st - 1] = push_vec(h, la);
-    for (int d = 0; d < 3; ++d) o_bc[st - 1][d] = push_vec(h, bc[d]);
+    o_bc[st - 1] = push_vec(h, bc);
     o_c2p[st - 1] = push_vec(h, ca);
   }
   // batched RKL2 stages (src/sts.hpp:111-157 per member): the state buffers of stage j rotate
   // as in the reference, the same way for every member, so their tables are fixed
   size_t o_span_s = 0, o_sts_c2p[4] = {}, o_sts_diff[4] = {}, o_sts_res[4] = {}, o_sts_div[2] = {}, o_sts_comb[5] = {},
-         o_sts_bc[4][3] = {}, o_sts_zero = 0, o_sts_copy0 = 0;
+         o_sts_bc[4] = {}, o_sts_zero = 0, o_sts_copy0 = 0;
   if (B->sts) {
     cudaError_t e0 = cudaMalloc(&B->sts_skip, sizeof(int) * (size_t)n);
     if (e0 == cudaSuccess) e0 = cudaMemset(B->sts_skip, 0, sizeof(int) * (size_t)n);
@@ -1657,14 +1636,9 @@ int batch_build(chq_batch *B) {
       o_sts_c2p[b] = push_vec(h, c2);
       o_sts_diff[b] = push_vec(h, df);
       o_sts_res[b] = push_vec(h, rs);
-      for (int d = 0; d < 3; ++d) {
-        for (int j = 0; j < n; ++j) {
-          bb[j] = bc_args(J[j], 0, B->sts_skip + j, d);
-          bb[j].u = U(J[j], b);
-          bb[j].b1 = BF(J[j], b, 0); bb[j].b2 = BF(J[j], b, 1); bb[j].b3 = BF(J[j], b, 2);
-        }
-        o_sts_bc[b][d] = push_vec(h, bb);
-      }
+      for (int j = 0; j < n; ++j)
+        bb[j] = bc_args_ptr(J[j], U(J[j], b), BF(J[j], b, 0), BF(J[j], b, 1), BF(J[j], b, 2), B->sts_skip + j);
+      o_sts_bc[b] = push_vec(h, bb);
     }
     for (int v = 0; v < 2; ++v) {   // M0 (first stage) or Mj
       for (int j = 0; j < n; ++j) {
@@ -1750,7 +1724,7 @@ int batch_build(chq_batch *B) {
   B->k_flag.slots = (BatchSlot *)(d + o_flag_s);
   B->k_repair.slots = (BatchSlot *)(d + o_repair_s);
   B->k_limit.slots = (BatchSlot *)(d + o_limit_s);
-  for (int q = 0; q < 3; ++q) B->k_bc[q].slots = (BatchSlot *)(d + o_bc_s[q]);
+  B->k_bc.slots = (BatchSlot *)(d + o_bc_s);
   B->k_c2p.slots = (BatchSlot *)(d + o_c2p_s);
   B->a_corner = d + o_corner;
   B->a_corner_need = d + o_corner_need;
@@ -1765,14 +1739,14 @@ int batch_build(chq_batch *B) {
   B->a_cool = d + o_cool;
   B->a_c2p_split[0] = d + o_split0;
   B->a_c2p_split[1] = d + o_split1;
-  for (int q = 0; q < 3; ++q) B->a_bc0[q] = d + o_bc0[q];
+  B->a_bc0 = d + o_bc0;
   if (B->sts) {
     B->k_span.slots = (BatchSlot *)(d + o_span_s);
     for (int b = 0; b < 4; ++b) {
       B->a_sts_c2p[b] = d + o_sts_c2p[b];
       B->a_sts_diff[b] = d + o_sts_diff[b];
       B->a_sts_res[b] = d + o_sts_res[b];
-      for (int q = 0; q < 3; ++q) B->a_sts_bc[b][q] = d + o_sts_bc[b][q];
+      B->a_sts_bc[b] = d + o_sts_bc[b];
     }
     for (int v = 0; v < 2; ++v) B->a_sts_div[v] = d + o_sts_div[v];
     for (int v = 0; v < 5; ++v) B->a_sts_comb[v] = d + o_sts_comb[v];
@@ -1789,7 +1763,7 @@ int batch_build(chq_batch *B) {
     B->a_flag[st] = d + o_flag[st];
     B->a_repair[st] = d + o_repair[st];
     B->a_limit[st] = d + o_limit[st];
-    for (int q = 0; q < 3; ++q) B->a_bc[st][q] = d + o_bc[st][q];
+    B->a_bc[st] = d + o_bc[st];
     B->a_c2p[st] = d + o_c2p[st];
   }
   return CHQ_OK;
@@ -1888,49 +1862,45 @@ int batch_sts(chq_batch *B, cudaStream_t s, long long &L) {
   const double *coef_dev = reinterpret_cast<const double *>(B->sts_dyn + o_coef);
   const dim3 b2(32, 8);
   const unsigned nspan = (unsigned)B->k_span.nblocks;
-  span_batched<<<nspan, 256, 0, s>>>((const SpanArgs *)B->a_sts_copy0, B->k_span.slots, n);
+  pdl(span_batched, nspan, 256, 0, s, (const SpanArgs *)B->a_sts_copy0, B->k_span.slots, n);
   CHQ_CUDA(cudaGetLastError());
   ++L;
   for (int st = 1; st <= smax; ++st) {
     const int bi = wrote(st - 1), bo = wrote(st);
     const int form = st == 1 ? 0 : st == 2 ? 1 : 2 + (st % 3);
-    sts_skip_kernel<<<(n + 127) / 128, 128, 0, s>>>(B->sts_skip, nst_dev, n, st);
-    c2p_batched<P><<<(unsigned)B->k_c2p.nblocks, b2, 0, s>>>((const C2pArgs<P> *)B->a_sts_c2p[bi], B->k_c2p.slots, n);
-    span_batched<<<nspan, 256, 0, s>>>((const SpanArgs *)B->a_sts_zero, B->k_span.slots, n);
+    pdl(sts_skip_kernel, (n + 127) / 128, 128, 0, s, B->sts_skip, nst_dev, n, st);
+    pdl(c2p_batched<P>, (unsigned)B->k_c2p.nblocks, b2, 0, s, (const C2pArgs<P> *)B->a_sts_c2p[bi], B->k_c2p.slots, n);
+    pdl(span_batched, nspan, 256, 0, s, (const SpanArgs *)B->a_sts_zero, B->k_span.slots, n);
     CHQ_CUDA(cudaGetLastError());
     L += 3;
     if (B->k_diff.nblocks) {
-      diff_flux_batched<P><<<(unsigned)B->k_diff.nblocks, 256, 0, s>>>((const DiffArgs<P> *)B->a_sts_diff[bi],
+      pdl(diff_flux_batched<P>, (unsigned)B->k_diff.nblocks, 256, 0, s, (const DiffArgs<P> *)B->a_sts_diff[bi],
                                                                         B->k_diff.slots, n);
       ++L;
     }
     if (B->k_res.nblocks) {
-      resistive_emf_batched<P><<<(unsigned)B->k_res.nblocks, b2, 0, s>>>((const ResEmfArgs<P> *)B->a_sts_res[bi],
+      pdl(resistive_emf_batched<P>, (unsigned)B->k_res.nblocks, b2, 0, s, (const ResEmfArgs<P> *)B->a_sts_res[bi],
                                                                          B->k_res.slots, n);
       ++L;
     }
-    sts_div_batched<P><<<(unsigned)B->k_update.nblocks, b2, 0, s>>>((const StsDivArgs<P> *)B->a_sts_div[st == 1 ? 0 : 1],
+    pdl(sts_div_batched<P>, (unsigned)B->k_update.nblocks, b2, 0, s, (const StsDivArgs<P> *)B->a_sts_div[st == 1 ? 0 : 1],
                                                                       B->k_update.slots, n);
-    sts_combine_batched<<<(unsigned)B->k_update.nblocks, b2, 0, s>>>((const StsCombArgs *)B->a_sts_comb[form],
+    pdl(sts_combine_batched, (unsigned)B->k_update.nblocks, b2, 0, s, (const StsCombArgs *)B->a_sts_comb[form],
                                                                       B->k_update.slots, n,
                                                                       coef_dev + 5 * (size_t)(st - 1) * n);
     CHQ_CUDA(cudaGetLastError());
     L += 2;
-    if (B->k_bc[0].nblocks) bc_batched<0><<<(unsigned)B->k_bc[0].nblocks, 256, 0, s>>>((const BcArgs *)B->a_sts_bc[bo][0], B->k_bc[0].slots, n);
-    if (B->k_bc[1].nblocks) bc_batched<1><<<(unsigned)B->k_bc[1].nblocks, 256, 0, s>>>((const BcArgs *)B->a_sts_bc[bo][1], B->k_bc[1].slots, n);
-    if (B->k_bc[2].nblocks) bc_batched<2><<<(unsigned)B->k_bc[2].nblocks, 256, 0, s>>>((const BcArgs *)B->a_sts_bc[bo][2], B->k_bc[2].slots, n);
+    pdl(bc_batched, (unsigned)B->k_bc.nblocks, 256, 0, s, (const BcArgs *)B->a_sts_bc[bo], B->k_bc.slots, n);
     CHQ_CUDA(cudaGetLastError());
-    L += (B->k_bc[0].nblocks > 0) + (B->k_bc[1].nblocks > 0) + (B->k_bc[2].nblocks > 0);
+    L += 1;
   }
-  span_batched<<<nspan, 256, 0, s>>>((const SpanArgs *)(B->sts_dyn + o_fin), B->k_span.slots, n);
+  pdl(span_batched, nspan, 256, 0, s, (const SpanArgs *)(B->sts_dyn + o_fin), B->k_span.slots, n);
   CHQ_CUDA(cudaGetLastError());
   ++L;
   // the boundaries of the result in u0 / b?f0 (src/main.cpp:280)
-  if (B->k_bc[0].nblocks) bc_batched<0><<<(unsigned)B->k_bc[0].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc0[0], B->k_bc[0].slots, n);
-  if (B->k_bc[1].nblocks) bc_batched<1><<<(unsigned)B->k_bc[1].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc0[1], B->k_bc[1].slots, n);
-  if (B->k_bc[2].nblocks) bc_batched<2><<<(unsigned)B->k_bc[2].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc0[2], B->k_bc[2].slots, n);
+  pdl(bc_batched, (unsigned)B->k_bc.nblocks, 256, 0, s, (const BcArgs *)B->a_bc0, B->k_bc.slots, n);
   CHQ_CUDA(cudaGetLastError());
-  L += (B->k_bc[0].nblocks > 0) + (B->k_bc[1].nblocks > 0) + (B->k_bc[2].nblocks > 0);
+  L += 1;
   return CHQ_OK;
 }
 
@@ -1940,74 +1910,63 @@ int batch_cycle(chq_batch *B, cudaStream_t s) {
   const int n = (int)B->jobs.size();
   const dim3 b2(32, 8);
   long long &L = B->nlaunch;
-  ctl_begin_batched<<<(n + 127) / 128, 128, 0, s>>>(B->ctls, n);
+  pdl(ctl_begin_batched, (n + 127) / 128, 128, 0, s, B->ctls, n);
   CHQ_CUDA(cudaGetLastError());
   ++L;
   for (int st = 0; st < B->nstage; ++st) {
     CHQ_CUDA(batch_flux<P>(B, (const FluxArgs<P> *)B->a_flux[st], s));
     ++L;
     if (B->diff && B->k_diff.nblocks) {
-      diff_flux_batched<P><<<(unsigned)B->k_diff.nblocks, 256, 0, s>>>((const DiffArgs<P> *)B->a_diff[st], B->k_diff.slots, n);
+      pdl(diff_flux_batched<P>, (unsigned)B->k_diff.nblocks, 256, 0, s, (const DiffArgs<P> *)B->a_diff[st], B->k_diff.slots, n);
       CHQ_CUDA(cudaGetLastError());
       ++L;
     }
     if (B->limiter && B->k_limit.nblocks) {
-      limit_batched<P><<<(unsigned)B->k_limit.nblocks, 256, 0, s>>>((const LimitArgs<P> *)B->a_limit[st], B->k_limit.slots, n);
+      pdl(limit_batched<P>, (unsigned)B->k_limit.nblocks, 256, 0, s, (const LimitArgs<P> *)B->a_limit[st], B->k_limit.slots, n);
       CHQ_CUDA(cudaGetLastError());
       ++L;
     }
     auto update = [&](const void *args) -> cudaError_t {
       if (B->grav)
-        update_batched<P, true><<<(unsigned)B->k_update.nblocks, b2, 0, s>>>((const UpdateArgs<P> *)args, B->k_update.slots, n);
+        pdl(update_batched<P, true>, (unsigned)B->k_update.nblocks, b2, 0, s, (const UpdateArgs<P> *)args, B->k_update.slots, n);
       else
-        update_batched<P, false><<<(unsigned)B->k_update.nblocks, b2, 0, s>>>((const UpdateArgs<P> *)args, B->k_update.slots, n);
+        pdl(update_batched<P, false>, (unsigned)B->k_update.nblocks, b2, 0, s, (const UpdateArgs<P> *)args, B->k_update.slots, n);
       ++L;
       return cudaGetLastError();
     };
     auto res_emf = [&](const void *args) -> cudaError_t {
       if (!B->diff || !B->k_res.nblocks) return cudaSuccess;
-      resistive_emf_batched<P><<<(unsigned)B->k_res.nblocks, b2, 0, s>>>((const ResEmfArgs<P> *)args, B->k_res.slots, n);
+      pdl(resistive_emf_batched<P>, (unsigned)B->k_res.nblocks, b2, 0, s, (const ResEmfArgs<P> *)args, B->k_res.slots, n);
       ++L;
       return cudaGetLastError();
     };
-    corner_emf_batched<P><<<(unsigned)B->k_corner.nblocks, b2, 0, s>>>((const EmfArgs<P> *)B->a_corner, B->k_corner.slots, n);
+    pdl(corner_emf_batched<P>, (unsigned)B->k_corner.nblocks, b2, 0, s, (const EmfArgs<P> *)B->a_corner, B->k_corner.slots, n);
     CHQ_CUDA(cudaGetLastError());
     ++L;
     CHQ_CUDA(res_emf(B->a_res[st]));
     CHQ_CUDA(update(B->a_update[st]));
     if (B->fofc) {
-      fofc_flag_batched<<<(unsigned)B->k_flag.nblocks, b2, 0, s>>>((const FlagArgs *)B->a_flag[st], B->k_flag.slots, n);
+      pdl(fofc_flag_batched, (unsigned)B->k_flag.nblocks, b2, 0, s, (const FlagArgs *)B->a_flag[st], B->k_flag.slots, n);
       CHQ_CUDA(cudaGetLastError());
-      fofc_repair_batched<P><<<(unsigned)B->k_repair.nblocks, 256, 0, s>>>((const RepairArgs<P> *)B->a_repair[st], B->k_repair.slots, n);
+      pdl(fofc_repair_batched<P>, (unsigned)B->k_repair.nblocks, 256, 0, s, (const RepairArgs<P> *)B->a_repair[st], B->k_repair.slots, n);
       CHQ_CUDA(cudaGetLastError());
       // (with explicit diffusion eta J is added to every edge afterwards: every edge is redone)
       if (B->diff)
-        corner_emf_batched<P><<<(unsigned)B->k_corner.nblocks, b2, 0, s>>>((const EmfArgs<P> *)B->a_corner_need, B->k_corner.slots, n);
+        pdl(corner_emf_batched<P>, (unsigned)B->k_corner.nblocks, b2, 0, s, (const EmfArgs<P> *)B->a_corner_need, B->k_corner.slots, n);
       else
-        corner_rerun_batched<P><<<(unsigned)B->k_corner_rerun.nblocks, 256, 0, s>>>((const EmfArgs<P> *)B->a_corner_need, B->k_corner_rerun.slots, n);
+        pdl(corner_rerun_batched<P>, (unsigned)B->k_corner_rerun.nblocks, 256, 0, s, (const EmfArgs<P> *)B->a_corner_need, B->k_corner_rerun.slots, n);
       CHQ_CUDA(cudaGetLastError());
       L += 3;
       CHQ_CUDA(res_emf(B->a_res_need[st]));
       CHQ_CUDA(update(B->a_update_need[st]));
     }
-    bc_batched<0><<<(unsigned)B->k_bc[0].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc[st][0], B->k_bc[0].slots, n);
-    CHQ_CUDA(cudaGetLastError());
+    CHQ_CUDA(pdl(bc_batched, (unsigned)B->k_bc.nblocks, 256, 0, s, (const BcArgs *)B->a_bc[st], B->k_bc.slots, n));
     ++L;
-    if (B->k_bc[1].nblocks) {
-      bc_batched<1><<<(unsigned)B->k_bc[1].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc[st][1], B->k_bc[1].slots, n);
-      CHQ_CUDA(cudaGetLastError());
-      ++L;
-    }
-    if (B->k_bc[2].nblocks) {
-      bc_batched<2><<<(unsigned)B->k_bc[2].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc[st][2], B->k_bc[2].slots, n);
-      CHQ_CUDA(cudaGetLastError());
-      ++L;
-    }
-    c2p_batched<P><<<(unsigned)B->k_c2p.nblocks, b2, 0, s>>>((const C2pArgs<P> *)B->a_c2p[st], B->k_c2p.slots, n);
+    pdl(c2p_batched<P>, (unsigned)B->k_c2p.nblocks, b2, 0, s, (const C2pArgs<P> *)B->a_c2p[st], B->k_c2p.slots, n);
     CHQ_CUDA(cudaGetLastError());
     ++L;
     if (st == B->nstage - 1 && ((B->diff && !B->cool) || B->sts)) {
-      rho_min_batched<P><<<(unsigned)B->k_rho.nblocks, b2, 0, s>>>((const RhoMinArgs<P> *)B->a_rho, B->k_rho.slots, n);
+      pdl(rho_min_batched<P>, (unsigned)B->k_rho.nblocks, b2, 0, s, (const RhoMinArgs<P> *)B->a_rho, B->k_rho.slots, n);
       CHQ_CUDA(cudaGetLastError());
       ++L;
     }
@@ -2018,31 +1977,25 @@ int batch_cycle(chq_batch *B, cudaStream_t s) {
   }
   if (B->cool) {
     // operator-split cooling of u0 after the step (src/main.cpp:272-290)
-    c2p_batched<P><<<(unsigned)B->k_c2p.nblocks, b2, 0, s>>>((const C2pArgs<P> *)B->a_c2p_split[0], B->k_c2p.slots, n);
+    pdl(c2p_batched<P>, (unsigned)B->k_c2p.nblocks, b2, 0, s, (const C2pArgs<P> *)B->a_c2p_split[0], B->k_c2p.slots, n);
     CHQ_CUDA(cudaGetLastError());
-    cooling_batched<P><<<(unsigned)B->k_cool.nblocks, b2, 0, s>>>((const CoolArgs<P> *)B->a_cool, B->k_cool.slots, n);
+    pdl(cooling_batched<P>, (unsigned)B->k_cool.nblocks, b2, 0, s, (const CoolArgs<P> *)B->a_cool, B->k_cool.slots, n);
     CHQ_CUDA(cudaGetLastError());
     L += 2;
-    for (int q = 0; q < 3; ++q) {
-      if (!B->k_bc[q].nblocks) continue;
-      if (q == 0) bc_batched<0><<<(unsigned)B->k_bc[0].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc0[0], B->k_bc[0].slots, n);
-      if (q == 1) bc_batched<1><<<(unsigned)B->k_bc[1].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc0[1], B->k_bc[1].slots, n);
-      if (q == 2) bc_batched<2><<<(unsigned)B->k_bc[2].nblocks, 256, 0, s>>>((const BcArgs *)B->a_bc0[2], B->k_bc[2].slots, n);
-      CHQ_CUDA(cudaGetLastError());
-      ++L;
-    }
+    CHQ_CUDA(pdl(bc_batched, (unsigned)B->k_bc.nblocks, 256, 0, s, (const BcArgs *)B->a_bc0, B->k_bc.slots, n));
+    ++L;
   }
   if (B->cool || B->sts) {
-    c2p_batched<P><<<(unsigned)B->k_c2p.nblocks, b2, 0, s>>>((const C2pArgs<P> *)B->a_c2p_split[1], B->k_c2p.slots, n);
+    pdl(c2p_batched<P>, (unsigned)B->k_c2p.nblocks, b2, 0, s, (const C2pArgs<P> *)B->a_c2p_split[1], B->k_c2p.slots, n);
     CHQ_CUDA(cudaGetLastError());
     ++L;
     if (B->diff) {
-      rho_min_batched<P><<<(unsigned)B->k_rho.nblocks, b2, 0, s>>>((const RhoMinArgs<P> *)B->a_rho, B->k_rho.slots, n);
+      pdl(rho_min_batched<P>, (unsigned)B->k_rho.nblocks, b2, 0, s, (const RhoMinArgs<P> *)B->a_rho, B->k_rho.slots, n);
       CHQ_CUDA(cudaGetLastError());
       ++L;
     }
   }
-  ctl_end_batched<<<(n + 127) / 128, 128, 0, s>>>(B->ctls, n);
+  pdl(ctl_end_batched, (n + 127) / 128, 128, 0, s, B->ctls, n);
   CHQ_CUDA(cudaGetLastError());
   ++L;
   CHQ_CUDA(cudaGetLastError());
@@ -2593,7 +2546,7 @@ int chq_corner_emf(chq_mesh *m, void *stream) {
 
 int chq_update(chq_mesh *m, int out, double g0, double g1, double beta_dt, void *stream) {
   if (!m || (out != 0 && out != 1)) return fail(CHQ_ERR_ARG, "bad argument");
-  return DISPATCH_P(m, do_update)(m, out, g0, g1, beta_dt, nullptr, nullptr, nullptr, S(m, stream));
+  return DISPATCH_P(m, do_update)(m, out, g0, g1, beta_dt, nullptr, nullptr, S(m, stream));
 }
 
 int chq_boundaries(chq_mesh *m, int buf, void *stream) {
@@ -2692,10 +2645,10 @@ int plain_cycles(chq_mesh *m, int n, cudaStream_t s) {
   for (int c = 0; c < n; ++c) {
     {
       Prof p(m, PK_CTL, s);
-      ctl_begin_kernel<<<1, 1, 0, s>>>(m->ctl, 0);
+      pdl(ctl_begin_kernel, 1, 1, 0, s, m->ctl, 0);
       m->nlaunch += 1;
       if (m->hrec) {
-        hst_due_kernel<<<1, 1, 0, s>>>(m->ctl, m->hrec);
+        pdl(hst_due_kernel, 1, 1, 0, s, m->ctl, m->hrec);
         m->nlaunch += 1;
       }
     }
@@ -2755,11 +2708,11 @@ int plain_cycles(chq_mesh *m, int n, cudaStream_t s) {
     }
     {
       Prof p(m, PK_CTL, s);
-      ctl_end_kernel<<<1, 1, 0, s>>>(m->ctl);
+      pdl(ctl_end_kernel, 1, 1, 0, s, m->ctl);
       m->nlaunch += 1;
       if (m->hrec) {
-        hst_fold_kernel<<<(unsigned)m->hrec_nfold, 320, 0, s>>>(m->hrec);
-        hst_commit_kernel<<<1, 320, 0, s>>>(m->ctl, m->hrec);
+        pdl(hst_fold_kernel, (unsigned)m->hrec_nfold, 320, 0, s, m->hrec);
+        pdl(hst_commit_kernel, 1, 320, 0, s, m->ctl, m->hrec);
         m->nlaunch += 2;
       }
     }
@@ -3726,7 +3679,7 @@ int chq_slab_prime(chq_mesh *m, double t, int part, void *stream) {
 int chq_slab_begin(chq_mesh *m, void *stream) {
   if (int rc = slab_check(m)) return rc;
   cudaStream_t s = S(m, stream);
-  ctl_begin_kernel<<<1, 1, 0, s>>>(m->ctl, 0);
+  pdl(ctl_begin_kernel, 1, 1, 0, s, m->ctl, 0);
   CHQ_CUDA(cudaGetLastError());
   m->nlaunch += 1;
   return CHQ_OK;
@@ -3756,7 +3709,7 @@ int chq_slab_stage(chq_mesh *m, int stage, int part, void *stream) {
 int chq_slab_end(chq_mesh *m, void *stream) {
   if (int rc = slab_check(m)) return rc;
   cudaStream_t s = S(m, stream);
-  ctl_end_kernel<<<1, 1, 0, s>>>(m->ctl);
+  pdl(ctl_end_kernel, 1, 1, 0, s, m->ctl);
   CHQ_CUDA(cudaGetLastError());
   m->nlaunch += 1;
   return CHQ_OK;
