@@ -266,17 +266,20 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_kern
 // FOFC re-run of the whole update: every point of the frame, blocks striding over its 32 x 8
 // tiles. A bounded grid, because the launch mostly has nothing to do, and the update's own grid
 // (76 000 blocks at 256^3) takes some 25 us a stage just to start and return.
-template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_rerun_kernel(const UpdateArgs<P> A) {
-  pdl_begin();
+template <class P, bool GRAV> CHQ_D void update_rerun_body(const UpdateArgs<P> &A, int b, int nb) {
   if (A.done && *A.done) return;
   if (*A.need <= A.need_min) return;
   const Geom &g = A.g;
   const int nx = (g.ie + 2 - g.is + 31) / 32, ny = (g.je + 2 - g.js + 7) / 8, nz = g.ke + 2 - g.ks;
   const long tiles = (long)nx * ny * nz;
-  for (long t = blockIdx.x; t < tiles; t += gridDim.x) {
+  for (long t = b; t < tiles; t += nb) {
     const long r = t / nx;
     update_body<P, GRAV>(A, (int)(t - r * nx), (int)(r % ny), (int)(r / ny));
   }
+}
+template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_rerun_kernel(const UpdateArgs<P> A) {
+  pdl_begin();
+  update_rerun_body<P, GRAV>(A, blockIdx.x, gridDim.x);
 }
 
 // FOFC re-run of the update in a stage whose b-weight is zero and whose output is the
@@ -387,16 +390,16 @@ CHQ_D void fofc_flag_body(const FlagArgs &A, int bx, int by, int bz) {
     const double bx = 0.5 * (A.b1[l] + A.b1[l + 1]);
     const double by = g.two_d ? 0.5 * (A.b2[l] + A.b2[l + g.sj]) : A.b2[l];
     const double bz = g.three_d ? 0.5 * (A.b3[l] + A.b3[l + g.sk]) : A.b3[l];
-    const double d = A.u[IDN * vs + l];
-    bool b = (d <= A.eos.dfloor);
-    if (!b) {
-      const double ke = divz(0.5 * (sqr(A.u[IM1 * vs + l]) + sqr(A.u[IM2 * vs + l]) + sqr(A.u[IM3 * vs + l])), d);
-      const double eint = A.u[IEN * vs + l] - ke - 0.5 * (bx * bx + by * by + bz * bz);
-      double p = A.eos.gm1 * eint;
-      if (A.eos.dual_energy && eint < A.eos.de_eta * fabs(A.u[IEN * vs + l]))
-        p = (A.u[IENT * vs + l] / d) * pow(d, A.eos.gamma);
-      b = (p <= A.eos.pfloor);
-    }
+    // every load before the first test: the loads behind a branch cost the cell a second round
+    // trip to memory (at 256^3 231 -> 181 us, 4.9 -> 6.3 TB/s)
+    const double d = A.u[IDN * vs + l], m1 = A.u[IM1 * vs + l], m2 = A.u[IM2 * vs + l], m3 = A.u[IM3 * vs + l];
+    const double en = A.u[IEN * vs + l];
+    const double mm = 0.5 * (sqr(m1) + sqr(m2) + sqr(m3));
+    const double ke = in_range(d) ? quot(mm, d, rcp_a(d)) : divz(mm, d);
+    const double eint = en - ke - 0.5 * (bx * bx + by * by + bz * bz);
+    double p = A.eos.gm1 * eint;
+    if (A.eos.dual_energy && eint < A.eos.de_eta * fabs(en)) p = (A.u[IENT * vs + l] / d) * pow(d, A.eos.gamma);
+    const bool b = (d <= A.eos.dfloor) || (p <= A.eos.pfloor);
     bad = b ? 1 : 0;
     A.flag[l] = bad;
   }
@@ -884,7 +887,7 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
     const double bz = g.three_d ? 0.5 * (A.b3[l] + A.b3[l + g.sk]) : A.b3[l];
     const EOSp &e = A.eos;
     const double d = fmax(A.u[IDN * vs + l], e.dfloor);
-    const double id = 1.0 / d;
+    const double id = in_range(d) ? rcp_rn(d) : 1.0 / d;
     const double vx = A.u[IM1 * vs + l] * id, vy = A.u[IM2 * vs + l] * id, vz = A.u[IM3 * vs + l] * id;
     const double bsq = bx * bx + by * by + bz * bz;
     const double ke = 0.5 * d * (vx * vx + vy * vy + vz * vz);
@@ -900,7 +903,8 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
       A.u[IEN * vs + l] = en;
     } else {
       p = fmax(p, e.pfloor);
-      sent = p / pow(d, e.gamma);
+      const double dg = pow(d, e.gamma);
+      sent = in_range(dg) ? quot(p, dg, rcp_a(dg)) : p / dg;
       A.u[IENT * vs + l] = d * sent;
     }
     A.w[IDN * vs + l] = P(d);
@@ -918,13 +922,19 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
     if (A.compute_dt && i >= g.is && i <= g.ie && j >= g.js && j <= g.je && k >= g.ks && k <= g.ke) {
       const double gp = e.gamma * p;
       const double a = (gp + bsq) * id;
-      auto cf = [&](double bn) {
+      const bool ok = in_range(a);
+      auto dt_of = [&](double dx, double v, double bn) {   // dx / (|v| + fast speed along the axis)
         const double disc = a * a - 4.0 * gp * bn * bn * id * id;
-        return sqrt(0.5 * (a + sqrt(fmax(disc, 0.0))));
+        if (ok) {
+          const double root = sqrt_q(disc);
+          const double s = fabs(v) + sqrt_q(0.5 * (a + (disc > RootFloor<double>::v ? root : 0.0)));
+          if (in_range(s)) return quot(dx, s, rcp_a(s));
+        }
+        return dx / (fabs(v) + sqrt(0.5 * (a + sqrt(fmax(disc, 0.0)))));
       };
-      double dt = g.dx1 / (fabs(vx) + cf(bx));
-      if (g.two_d) dt = fmin(dt, g.dx2 / (fabs(vy) + cf(by)));
-      if (g.three_d) dt = fmin(dt, g.dx3 / (fabs(vz) + cf(bz)));
+      double dt = dt_of(g.dx1, vx, bx);
+      if (g.two_d) dt = fmin(dt, dt_of(g.dx2, vy, by));
+      if (g.three_d) dt = fmin(dt, dt_of(g.dx3, vz, bz));
       mdt = dt;
     }
     if (hdue && i >= g.is && i <= g.ie && j >= g.js && j <= g.je && k >= g.ks && k <= g.ke) {
@@ -988,8 +998,11 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
   }
 }
 
+// 6 blocks per SM (40 registers): the pow of the entropy and the quotients are a long chain a
+// cell, which more warps hide better than registers: 646 us (60 registers) and 642 / 628 / 611 us
+// with 4 / 5 / 6 blocks a launch at 256^3 in FP64 (5.2 TB/s), mixed 549 -> 505 us.
 template <class P, bool HST = false>
-__global__ void __launch_bounds__(256) c2p_kernel(const C2pArgs<P> A) { pdl_begin(); c2p_body<P, HST>(A, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void __launch_bounds__(256, 6) c2p_kernel(const C2pArgs<P> A) { pdl_begin(); c2p_body<P, HST>(A, blockIdx.x, blockIdx.y, blockIdx.z); }
 
 // Output test of the cycle just begun: its end time t + dt reaches the next output time
 // (the driver's check after t += dt, src/main.cpp:212-223).
@@ -1071,6 +1084,13 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_batc
   __shared__ __align__(16) unsigned char sa[sizeof(UpdateArgs<P>)];
   const UpdateArgs<P> &A = stage_args(args, j, sa);
   update_body<P, GRAV>(A, bx, by, bz);
+}
+template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_rerun_batched(const UpdateArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
+  const int j = batch_job(slots, n, blockIdx.x);
+  __shared__ __align__(16) unsigned char sa[sizeof(UpdateArgs<P>)];
+  const UpdateArgs<P> &A = stage_args(args, j, sa);
+  update_rerun_body<P, GRAV>(A, (int)(blockIdx.x - slots[j].off), slots[j].gx);
 }
 __global__ void __launch_bounds__(256) fofc_flag_batched(const FlagArgs *args, const BatchSlot *slots, int n) {
   pdl_begin();

@@ -204,6 +204,7 @@ struct chq_mesh {
   int lo[3][3], hi[3][3], active[3];
   int act_lo[3][3], act_hi[3][3];
   int seglen;
+  bool march_set = false;   // set by the caller or a tuner (a batch then keeps it)
   int xvar = 0;   // x-sweep kernel variant (register cap), chq_autotune
   // y/z staging of the FP64 streaming-PPM march: 0 cp.async, 1 TMA (chq_autotune_yz); the
   // tensor maps over w and bcc are encoded at creation when the driver offers the encoder
@@ -395,18 +396,19 @@ YzShape yz_shape(const chq_mesh *m, int d, int len) {
 // 0.6 of a face's work), and the launch runs in waves of the resident blocks: the length with
 // the least waves x (length + 0.6). Small meshes thus take one face a thread (OT 64^2: 22 us a
 // flux launch at length 4, the old rule's), large ones the longest march.
-int default_march(const chq_mesh *m) {
-  const double resident = 148.0 * (m->mixed ? 6 : 3);   // y/z blocks of the PPM kernels (FluxYzMinBlocks)
+int default_march(chq_mesh *const *ms, size_t n) {
+  const double resident = 148.0 * (ms[0]->mixed ? 6 : 3);   // y/z blocks of the PPM kernels (FluxYzMinBlocks)
   int best = 4;
   double least = 1e300;
   for (int L : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64}) {
     double blocks = 0.0, len = 1.0;
-    for (int d = 1; d < 3; ++d) {
-      if (!m->active[d]) continue;
-      const YzShape y = yz_shape(m, d, L);
-      blocks += (double)((y.ncol + kYzThreads - 1) / kYzThreads) * y.nseg;
-      len = std::max(len, (double)y.slen);
-    }
+    for (size_t q = 0; q < n; ++q)
+      for (int d = 1; d < 3; ++d) {
+        if (!ms[q]->active[d]) continue;
+        const YzShape y = yz_shape(ms[q], d, L);
+        blocks += (double)((y.ncol + kYzThreads - 1) / kYzThreads) * y.nseg;
+        len = std::max(len, (double)y.slen);
+      }
     const double waves = (blocks < 4.0 * resident) ? std::ceil(blocks / resident) : blocks / resident + 0.5;
     const double cost = std::max(waves, 1.0) * (len + 0.6);
     if (cost < 0.999 * least) {
@@ -418,7 +420,7 @@ int default_march(const chq_mesh *m) {
 }
 
 template <class P>
-FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask) {
+FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask, int march = 0) {
   FluxArgs<P> a{};
   a.g = m->g;
   a.eos = m->eos;
@@ -451,7 +453,7 @@ FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask) {
   const long places = (long)a.nxent * a.nxrow;
   a.nxwarp = a.active[0] ? (int)std::max(1L, (places - (32 - per) + per - 1) / per) : 0;
   for (int d = 1; d < 3; ++d) {
-    const YzShape y = yz_shape(m, d, m->seglen);
+    const YzShape y = yz_shape(m, d, march > 0 ? march : m->seglen);
     a.slen[d] = y.slen;
     a.nseg[d] = y.nseg;
     a.ncol[d] = y.ncol;
@@ -1420,7 +1422,7 @@ struct chq_batch {
   // the update epilogue; cooling is split after the step
   int diff = 0, grav = 0, cool = 0;
   int sts = 0;   // RKL2 members: super-time-stepping stages batched after the hyperbolic stages
-  Kind k_diff, k_res, k_rho, k_cool, k_corner_rerun;
+  Kind k_diff, k_res, k_rho, k_cool, k_corner_rerun, k_rerun;
   // batched RKL2 stages: argument tables per state buffer (Y0, Y1, Y2, u1) and per stage form,
   // built once; stage counts, coefficients and the final copies are uploaded every cycle
   Kind k_span;
@@ -1481,17 +1483,26 @@ int batch_build(chq_batch *B) {
   HostTable h;
   const std::vector<chq_mesh *> &J = B->jobs;
   const int n = (int)J.size();
+  // the members fill the device together, so the march length is chosen for all of them (a
+  // mesh's own default spreads it over the whole device), unless one was set or tuned
+  bool set = false;
+  for (const chq_mesh *m : J) set = set || m->march_set;
+  const int march = set ? 0 : default_march(J.data(), J.size());
   size_t o_flux_s, o_corner_s, o_update_s, o_flag_s, o_repair_s, o_limit_s, o_bc_s, o_c2p_s;
   o_flux_s = slots_of(h, J, [](chq_mesh *m) {
     const FluxArgs<P> a = flux_args<P>(m, 0, 7u);
     return linear((long)a.nxwarp * 32, 128);
   }, B->k_flux.nblocks);
-  const size_t o_flux_yz_s = slots_of(h, J, [](chq_mesh *m) {
-    const FluxArgs<P> a = flux_args<P>(m, 0, 7u);
+  const size_t o_flux_yz_s = slots_of(h, J, [march](chq_mesh *m) {
+    const FluxArgs<P> a = flux_args<P>(m, 0, 7u, march);
     return linear((long)(a.nblk[1] + a.nblk[2]) * kYzThreads, kYzThreads);
   }, B->k_flux_yz.nblocks);
   o_corner_s = slots_of(h, J, [](chq_mesh *m) { return corner_grid(m); }, B->k_corner.nblocks);
   o_update_s = slots_of(h, J, [](chq_mesh *m) { return update_grid(m); }, B->k_update.nblocks);
+  const size_t o_rerun_s = slots_of(h, J, [](chq_mesh *m) {
+    const Launch3 L = update_grid(m);
+    return Launch3{dim3((unsigned)std::min((long)L.grid.x * L.grid.y * L.grid.z, kRepairBlocksBatched)), dim3(32, 8)};
+  }, B->k_rerun.nblocks);
   o_flag_s = slots_of(h, J, [](chq_mesh *m) { return flag_grid(m); }, B->k_flag.nblocks);
   o_repair_s = slots_of(h, J, [](chq_mesh *m) {
     long tot = 0;
@@ -1573,7 +1584,7 @@ int batch_build(chq_batch *B) {
       da[j] = diff_args<P>(m, bc1, bc2, bc3, &c->done, nd);
       ea[j] = res_emf_args<P>(m, bc1, bc2, bc3, &c->done, nullptr);
       ean[j] = res_emf_args<P>(m, bc1, bc2, bc3, &c->done, &c->nbad);
-      fa[j] = flux_args<P>(m, cur, 7u);
+      fa[j] = flux_args<P>(m, cur, 7u, march);
       fa[j].skip = &c->done;
       ua[j] = update_args<P>(m, out, g0, g1, 0.0, &c->beta_dt[st - 1], &c->done, nullptr);
       uan[j] = update_args<P>(m, out, g0, g1, 0.0, &c->beta_dt[st - 1], &c->done, &c->nbad);
@@ -1721,6 +1732,7 @@ int batch_build(chq_batch *B) {
   B->k_flux_yz.slots = (BatchSlot *)(d + o_flux_yz_s);
   B->k_corner.slots = (BatchSlot *)(d + o_corner_s);
   B->k_update.slots = (BatchSlot *)(d + o_update_s);
+  B->k_rerun.slots = (BatchSlot *)(d + o_rerun_s);
   B->k_flag.slots = (BatchSlot *)(d + o_flag_s);
   B->k_repair.slots = (BatchSlot *)(d + o_repair_s);
   B->k_limit.slots = (BatchSlot *)(d + o_limit_s);
@@ -1958,7 +1970,10 @@ int batch_cycle(chq_batch *B, cudaStream_t s) {
       CHQ_CUDA(cudaGetLastError());
       L += 3;
       CHQ_CUDA(res_emf(B->a_res_need[st]));
-      CHQ_CUDA(update(B->a_update_need[st]));
+      const UpdateArgs<P> *again = (const UpdateArgs<P> *)B->a_update_need[st];
+      if (B->grav) CHQ_CUDA(pdl(update_rerun_batched<P, true>, (unsigned)B->k_rerun.nblocks, b2, 0, s, again, B->k_rerun.slots, n));
+      else CHQ_CUDA(pdl(update_rerun_batched<P, false>, (unsigned)B->k_rerun.nblocks, b2, 0, s, again, B->k_rerun.slots, n));
+      ++L;
     }
     CHQ_CUDA(pdl(bc_batched, (unsigned)B->k_bc.nblocks, 256, 0, s, (const BcArgs *)B->a_bc[st], B->k_bc.slots, n));
     ++L;
@@ -2195,7 +2210,7 @@ int mesh_create_impl(const chq_config *cfg, int nslab, int rank, chq_mesh **out)
   m->active[0] = 1;
   m->active[1] = g.two_d;
   m->active[2] = g.three_d;
-  m->seglen = default_march(m);
+  m->seglen = default_march(&m, 1);
 
   // one slab: doubles (u0, u1: 6 each; 6 face fields), P fields (w 6, bcc 3, ecc 3,
   // fluxes 18, face EMFs 6, edge EMFs 3), the int flag array, control block and scratch
@@ -3219,6 +3234,7 @@ int chq_set_seglen(chq_mesh *m, int seglen) {
   if (!m || seglen < 1 || seglen > 1024) return fail(CHQ_ERR_ARG, "march length must be in [1, 1024]");
   if (seglen != m->seglen) drop_cycle_graph(m);
   m->seglen = seglen;
+  m->march_set = true;
   return CHQ_OK;
 }
 
@@ -3341,6 +3357,7 @@ int chq_autotune2(chq_mesh *m, int *seglen, int *xvar, double ms_len[CHQ_TUNE_NL
     const auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
       m->seglen = it->second.first;
+      m->march_set = true;
       m->xvar = it->second.second;
       if (seglen) *seglen = m->seglen;
       if (xvar) *xvar = m->xvar;
@@ -3372,6 +3389,7 @@ int chq_autotune2(chq_mesh *m, int *seglen, int *xvar, double ms_len[CHQ_TUNE_NL
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune_cache[key] = {bl, bx};
   }
+  m->march_set = true;
   if (seglen) *seglen = bl;
   if (xvar) *xvar = bx;
   return CHQ_OK;
@@ -3451,12 +3469,13 @@ int chq_batch_autotune(chq_batch *B, int *seglen, int *xvar, double ms_len[CHQ_T
   // a new march length changes the flux launch geometry: rebuild the tables for it
   auto set = [&](int len, int v) -> int {
     bool same = (B->xvar == v);
-    for (const chq_mesh *m : B->jobs) same = same && (m->seglen == len);
+    for (const chq_mesh *m : B->jobs) same = same && m->march_set && (m->seglen == len);
     if (same && B->dev) return CHQ_OK;
     batch_free(B);
     for (chq_mesh *m : B->jobs) {
       if (m->seglen != len) drop_cycle_graph(m);
       m->seglen = len;
+      m->march_set = true;
       m->xvar = v;
     }
     B->xvar = v;

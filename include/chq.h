@@ -237,8 +237,9 @@ CHQ_API int chq_profile(chq_mesh *m, int enable);
  * members (their march lengths and the batch's x variant change together; the batch's tables
  * are rebuilt for each candidate) and caches per (precision, scheme, log2 of the batch's
  * cells, log2 of its member count); a batch of 2^23 cells or more fills the device with its
- * members' own settings and is returned untimed (the arrays hold -1). A batch starts with its
- * members' march lengths and its first member's x variant. */
+ * members' own settings and is returned untimed (the arrays hold -1). A batch starts with the
+ * march length that suits its members together, or with the members' own once one was set or
+ * tuned, and with its first member's x variant. */
 #define CHQ_TUNE_NLEN 5
 #define CHQ_TUNE_LENGTHS {4, 8, 16, 32, 64}
 #define CHQ_TUNE_NXVAR 2
