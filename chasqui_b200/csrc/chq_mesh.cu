@@ -514,11 +514,12 @@ EmfArgs<P> corner_args(chq_mesh *m, const int *done, const int *need) {
   return a;
 }
 
+// grid of a plane-wise kernel over nx x ny points of nz planes
+Launch3 plane_grid(int nx, int ny, int nz) { return {dim3((nx + 31) / 32, (ny + 7) / 8, nz), dim3(32, 8)}; }
+
 Launch3 corner_grid(const chq_mesh *m) {
   const Geom &g = m->g;
-  const int nxi = g.ie + 2 - g.is, nyj = g.je + 2 - g.js;
-  const int nzk = g.three_d ? g.ke + 2 - g.ks : 1;
-  return {dim3((nxi + 31) / 32, (nyj + 7) / 8, nzk), dim3(32, 8)};
+  return plane_grid(g.ie + 2 - g.is, g.je + 2 - g.js, g.three_d ? g.ke + 2 - g.ks : 1);
 }
 
 template <class P>
@@ -574,8 +575,13 @@ UpdateArgs<P> update_args(chq_mesh *m, int out, double g0, double g1, double bdt
 
 Launch3 update_grid(const chq_mesh *m) {
   const Geom &g = m->g;
-  const int nxi = g.ie + 2 - g.is, nyj = g.je + 2 - g.js, nzk = g.ke + 2 - g.ks;
-  return {dim3((nxi + 31) / 32, (nyj + 7) / 8, nzk), dim3(32, 8)};
+  return plane_grid(g.ie + 2 - g.is, g.je + 2 - g.js, g.ke + 2 - g.ks);
+}
+
+// the same frame with its upper plane below 3-D (the RKL2 kernels, which write faces there)
+Launch3 frame_grid(const chq_mesh *m) {
+  const Geom &g = m->g;
+  return plane_grid(g.ie + 2 - g.is, g.je + 2 - g.js, g.ke + 2 - g.ks);
 }
 
 template <class P>
@@ -634,7 +640,7 @@ FlagArgs flag_args(chq_mesh *m, int buf, int *nbad_dev, const int *done) {
 
 Launch3 flag_grid(const chq_mesh *m) {
   const Geom &g = m->g;
-  return {dim3((g.nx1 + 31) / 32, (g.je - g.js + 1 + 7) / 8, g.ke - g.ks + 1), dim3(32, 8)};
+  return plane_grid(g.nx1, g.je - g.js + 1, g.ke - g.ks + 1);
 }
 
 int do_flag(chq_mesh *m, int buf, int *nbad_dev, const int *done, cudaStream_t s) {
@@ -796,7 +802,7 @@ C2pArgs<P> c2p_args(chq_mesh *m, int buf, int compute_dt, unsigned long long *bi
 
 Launch3 c2p_grid(const chq_mesh *m) {
   const Geom &g = m->g;
-  return {dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8)};
+  return plane_grid(g.ni, g.nj, g.nk);
 }
 
 template <class P>
@@ -870,9 +876,11 @@ Launch3 active_grid(const chq_mesh *m) {
 
 // diffusive fluxes of every active direction in one launch (diffusion::Fluxes<0..2>)
 template <class P>
-int do_diff(chq_mesh *m, const double *b1, const double *b2, const double *b3, const int *done, cudaStream_t s) {
+int do_diff(chq_mesh *m, const double *b1, const double *b2, const double *b3, const int *done, cudaStream_t s,
+            int set) {
   long tot = 0;
-  const DiffArgs<P> a = diff_args<P>(m, b1, b2, b3, done, tot);
+  DiffArgs<P> a = diff_args<P>(m, b1, b2, b3, done, tot);
+  a.set = set;
   if (tot == 0) return CHQ_OK;
   m->nlaunch += 1;
   pdl(diff_flux_kernel<P>, (unsigned)((tot + 255) / 256), 256, 0, s, a);
@@ -908,9 +916,10 @@ Launch3 res_emf_grid(const chq_mesh *m) {
 // eta J added to the edge EMFs (diffusion::ResistiveEMF); a no-op without resistivity
 template <class P>
 int do_res_emf(chq_mesh *m, const double *b1, const double *b2, const double *b3, const int *done, const int *need,
-               cudaStream_t s) {
+               cudaStream_t s, int set) {
   if (!(m->cfg.eta > 0.0)) return CHQ_OK;
-  const ResEmfArgs<P> a = res_emf_args<P>(m, b1, b2, b3, done, need);
+  ResEmfArgs<P> a = res_emf_args<P>(m, b1, b2, b3, done, need);
+  a.set = set;
   m->nlaunch += 1;
   pdl(resistive_emf_kernel<P>, res_emf_grid(m).grid, dim3(32, 8), 0, s, a);
   CHQ_CUDA(cudaGetLastError());
@@ -998,7 +1007,7 @@ int run_stage_a(chq_mesh *m, int cur, int out, double g0, double g1, double bdt,
   }
   if (dstage) {
     Prof p(m, PK_DIFF, s);
-    if ((rc = DISPATCH_P(m, do_diff)(m, bc1, bc2, bc3, done, s))) return rc;
+    if ((rc = DISPATCH_P(m, do_diff)(m, bc1, bc2, bc3, done, s, 0))) return rc;
   }
   if (m->cfg.flux_limiter) {
     Prof p(m, PK_LIMIT, s);
@@ -1010,7 +1019,7 @@ int run_stage_a(chq_mesh *m, int cur, int out, double g0, double g1, double bdt,
   }
   if (dstage) {
     Prof p(m, PK_DIFF, s);
-    if ((rc = DISPATCH_P(m, do_res_emf)(m, bc1, bc2, bc3, done, nullptr, s))) return rc;
+    if ((rc = DISPATCH_P(m, do_res_emf)(m, bc1, bc2, bc3, done, nullptr, s, 0))) return rc;
   }
   {
     Prof p(m, PK_UPDATE, s);
@@ -1039,7 +1048,7 @@ int run_stage_b(chq_mesh *m, int cur, int out, double g0, double g1, double bdt,
     if (dstage) rc = DISPATCH_P(m, do_corner)(m, done, nbad, s);
     else rc = DISPATCH_P(m, do_corner_rerun)(m, done, nbad, s);
     if (rc) return rc;
-    if (dstage && (rc = DISPATCH_P(m, do_res_emf)(m, bc1, bc2, bc3, done, nbad, s))) return rc;
+    if (dstage && (rc = DISPATCH_P(m, do_res_emf)(m, bc1, bc2, bc3, done, nbad, s, 0))) return rc;
     if ((rc = DISPATCH_P(m, do_update_rerun)(m, out, g0, g1, bdt, bdt_dev, done, nbad, s))) return rc;
   }
   Prof p(m, PK_BC, s);
@@ -1067,8 +1076,6 @@ struct StsState {
   double *b[3];
 };
 
-// M(U, B) of (cell state whose primitives are in w, face fields b) into (mu, mb): zeroed
-// flux and EMF arrays, the diffusive fluxes, eta J, then -div F and -curl E (sts::Operator)
 // one launch for up to six whole-array copies or zero fills of one mesh
 int launch_spans(chq_mesh *m, const SpanArgs &a, cudaStream_t s) {
   long words = 0;
@@ -1080,11 +1087,18 @@ int launch_spans(chq_mesh *m, const SpanArgs &a, cudaStream_t s) {
   return CHQ_OK;
 }
 
+// first component the diffusive terms change: the momenta with viscosity, else the energy only
+int sts_first_component(const chq_mesh *m) { return m->cfg.nu > 0.0 ? IM1 : IEN; }
+
+// M(U, B) of (cell state whose primitives are in w, face fields b) into (mu, mb): the diffusive
+// fluxes, eta J, then -div F and -curl E (sts::Operator). clear: zero the flux and EMF arrays
+// first, as the reference does before every operator; nothing here reads what that clears, so
+// only the last operator of a cycle does it, for what the arrays hold afterwards.
 template <class P>
-int sts_operator(chq_mesh *m, double *const b[3], double *mu, double *const mb[3], cudaStream_t s) {
+int sts_operator(chq_mesh *m, double *const b[3], double *mu, double *const mb[3], bool clear, cudaStream_t s) {
   const Geom &g = m->g;
-  {
-    SpanArgs z{};   // the flux and EMF arrays start from zero (sts::Operator)
+  if (clear) {
+    SpanArgs z{};
     for (int d = 0; d < 3; ++d) {
       z.dst[d] = (unsigned long long *)m->flx[d];
       z.words[d] = NVAR * (long)g.vstride * (long)m->psize / 8;
@@ -1094,17 +1108,19 @@ int sts_operator(chq_mesh *m, double *const b[3], double *mu, double *const mb[3
     z.nspan = 6;
     if (int rc = launch_spans(m, z, s)) return rc;
   }
-  int rc = do_diff<P>(m, b[0], b[1], b[2], nullptr, s);
+  int rc = do_diff<P>(m, b[0], b[1], b[2], nullptr, s, 1);
   if (rc) return rc;
-  if ((rc = do_res_emf<P>(m, b[0], b[1], b[2], nullptr, nullptr, s))) return rc;
+  if ((rc = do_res_emf<P>(m, b[0], b[1], b[2], nullptr, nullptr, s, 1))) return rc;
   StsDivArgs<P> a{};
+  a.n0 = sts_first_component(m);
+  a.curl = m->cfg.eta > 0.0;
   a.g = g;
   a.f1 = as<P>(m->flx[0]); a.f2 = as<P>(m->flx[1]); a.f3 = as<P>(m->flx[2]);
   a.e1 = as<P>(m->e[0]); a.e2 = as<P>(m->e[1]); a.e3 = as<P>(m->e[2]);
   a.mu = mu;
   a.mb1 = mb[0]; a.mb2 = mb[1]; a.mb3 = mb[2];
   a.idx1 = 1.0 / g.dx1; a.idx2 = 1.0 / g.dx2; a.idx3 = 1.0 / g.dx3;
-  const Launch3 L = update_grid(m);
+  const Launch3 L = frame_grid(m);
   m->nlaunch += 1;
   pdl(sts_div_kernel<P>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
@@ -1117,12 +1133,13 @@ int sts_combine(chq_mesh *m, const StsState &out, double a, const StsState &x, d
                 double *const qb[3], cudaStream_t s) {
   StsCombArgs A{};
   A.g = m->g;
+  A.n0 = sts_first_component(m);
   A.a = a; A.b = b; A.c = c; A.d = d; A.e = e;
   A.out = out.u; A.x = x.u; A.y = y.u; A.z = z.u; A.p = p; A.q = q;
   for (int k = 0; k < 3; ++k) {
     A.bo[k] = out.b[k]; A.bx[k] = x.b[k]; A.by[k] = y.b[k]; A.bz[k] = z.b[k]; A.bp[k] = pb[k]; A.bq[k] = qb[k];
   }
-  const Launch3 L = update_grid(m);
+  const Launch3 L = frame_grid(m);
   m->nlaunch += 1;
   pdl(sts_combine_kernel, L.grid, L.block, 0, s, A);
   CHQ_CUDA(cudaGetLastError());
@@ -1138,14 +1155,16 @@ int sts_advance(chq_mesh *m, double tau, double dt_par, cudaStream_t s, int &nst
   nst = sts_stage_count(tau, dt_par);
   const int ns = nst;
   const double w1 = 4.0 / (double(ns) * ns + ns - 2.0);
-  StsState Y0{m->sy[0], {m->sb[0][0], m->sb[0][1], m->sb[0][2]}};
+  // Y0 is u0 itself: nothing writes it before the final copy but con2prim, whose entropy slot
+  // is already what it writes
+  StsState Y0{m->u[0], {m->bf[0][0], m->bf[0][1], m->bf[0][2]}};
   StsState Y1{m->sy[1], {m->sb[1][0], m->sb[1][1], m->sb[1][2]}};
   StsState Y2{m->sy[2], {m->sb[2][0], m->sb[2][1], m->sb[2][2]}};
   StsState spare{m->u[1], {m->bf[1][0], m->bf[1][1], m->bf[1][2]}};
   double *M0 = m->sm0, *Mj = m->smj;
   double *MB0[3] = {m->smb0[0], m->smb0[1], m->smb0[2]}, *MBj[3] = {m->smbj[0], m->smbj[1], m->smbj[2]};
   int rc;
-  // Y0 = (u0, b?f0) and, at the end, (u0, b?f0) = Y_s: whole arrays, one launch each
+  // at the end (u0, b?f0) = Y_s: whole arrays, one launch
   auto copy = [&](double *du, double *const db[3], const double *su, const double *const sb[3]) {
     SpanArgs c{};
     c.dst[0] = (unsigned long long *)du;
@@ -1159,10 +1178,9 @@ int sts_advance(chq_mesh *m, double tau, double dt_par, cudaStream_t s, int &nst
     c.nspan = 4;
     return launch_spans(m, c, s);
   };
-  if ((rc = copy(Y0.u, Y0.b, m->u[0], m->bf[0]))) return rc;
   if ((rc = launch_c2p<P>(m, c2p_args_ptr<P>(m, Y0.u, Y0.b[0], Y0.b[1], Y0.b[2], 0, nullptr, nullptr, nullptr), s)))
     return rc;
-  if ((rc = sts_operator<P>(m, Y0.b, M0, MB0, s))) return rc;
+  if ((rc = sts_operator<P>(m, Y0.b, M0, MB0, false, s))) return rc;
   const double mt1 = double(sts_b(1) * w1) * tau;
   if ((rc = sts_combine(m, Y1, 1.0, Y0, 0.0, Y0, 0.0, Y0, mt1, M0, MB0, 0.0, M0, MB0, s))) return rc;
   if ((rc = do_bc_ptr(m, Y1.u, Y1.b[0], Y1.b[1], Y1.b[2], nullptr, s))) return rc;
@@ -1176,7 +1194,7 @@ int sts_advance(chq_mesh *m, double tau, double dt_par, cudaStream_t s, int &nst
     if ((rc = launch_c2p<P>(m, c2p_args_ptr<P>(m, yjm1.u, yjm1.b[0], yjm1.b[1], yjm1.b[2], 0, nullptr, nullptr,
                                                nullptr), s)))
       return rc;
-    if ((rc = sts_operator<P>(m, yjm1.b, Mj, MBj, s))) return rc;
+    if ((rc = sts_operator<P>(m, yjm1.b, Mj, MBj, j == ns, s))) return rc;
     if ((rc = sts_combine(m, yj, mu, yjm1, nu, yjm2, 1.0 - mu - nu, Y0, mut * tau, Mj, MBj, gt * tau, M0, MB0, s)))
       return rc;
     if ((rc = do_bc_ptr(m, yj.u, yj.b[0], yj.b[1], yj.b[2], nullptr, s))) return rc;
@@ -1422,12 +1440,12 @@ struct chq_batch {
   // the update epilogue; cooling is split after the step
   int diff = 0, grav = 0, cool = 0;
   int sts = 0;   // RKL2 members: super-time-stepping stages batched after the hyperbolic stages
-  Kind k_diff, k_res, k_rho, k_cool, k_corner_rerun, k_rerun;
+  Kind k_diff, k_res, k_rho, k_cool, k_corner_rerun, k_rerun, k_frame;
   // batched RKL2 stages: argument tables per state buffer (Y0, Y1, Y2, u1) and per stage form,
   // built once; stage counts, coefficients and the final copies are uploaded every cycle
   Kind k_span;
   void *a_sts_c2p[4] = {}, *a_sts_diff[4] = {}, *a_sts_res[4] = {}, *a_sts_div[2] = {}, *a_sts_comb[5] = {},
-       *a_sts_bc[4] = {}, *a_sts_zero = nullptr, *a_sts_copy0 = nullptr;
+       *a_sts_bc[4] = {}, *a_sts_zero = nullptr;
   int *sts_skip = nullptr;   // per member: skip the current RKL2 stage
   char *sts_dyn = nullptr;   // per cycle: stage counts | coefficients | final copies
   size_t sts_dyn_bytes = 0;
@@ -1499,6 +1517,7 @@ int batch_build(chq_batch *B) {
   }, B->k_flux_yz.nblocks);
   o_corner_s = slots_of(h, J, [](chq_mesh *m) { return corner_grid(m); }, B->k_corner.nblocks);
   o_update_s = slots_of(h, J, [](chq_mesh *m) { return update_grid(m); }, B->k_update.nblocks);
+  const size_t o_frame_s = slots_of(h, J, [](chq_mesh *m) { return frame_grid(m); }, B->k_frame.nblocks);
   const size_t o_rerun_s = slots_of(h, J, [](chq_mesh *m) {
     const Launch3 L = update_grid(m);
     return Launch3{dim3((unsigned)std::min((long)L.grid.x * L.grid.y * L.grid.z, kRepairBlocksBatched)), dim3(32, 8)};
@@ -1615,7 +1634,7 @@ int batch_build(chq_batch *B) {
   // batched RKL2 stages (src/sts.hpp:111-157 per member): the state buffers of stage j rotate
   // as in the reference, the same way for every member, so their tables are fixed
   size_t o_span_s = 0, o_sts_c2p[4] = {}, o_sts_diff[4] = {}, o_sts_res[4] = {}, o_sts_div[2] = {}, o_sts_comb[5] = {},
-         o_sts_bc[4] = {}, o_sts_zero = 0, o_sts_copy0 = 0;
+         o_sts_bc[4] = {}, o_sts_zero = 0;
   if (B->sts) {
     cudaError_t e0 = cudaMalloc(&B->sts_skip, sizeof(int) * (size_t)n);
     if (e0 == cudaSuccess) e0 = cudaMemset(B->sts_skip, 0, sizeof(int) * (size_t)n);
@@ -1633,8 +1652,9 @@ int batch_build(chq_batch *B) {
     std::vector<StsDivArgs<P>> dv(n);
     std::vector<StsCombArgs> cb(n);
     std::vector<BcArgs> bb(n);
-    auto U = [](chq_mesh *m, int b) { return b < 3 ? m->sy[b] : m->u[1]; };
-    auto BF = [](chq_mesh *m, int b, int d) { return b < 3 ? m->sb[b][d] : m->bf[1][d]; };
+    // Y0 is u0 in place, as in sts_advance
+    auto U = [](chq_mesh *m, int b) { return b == 0 ? m->u[0] : b < 3 ? m->sy[b] : m->u[1]; };
+    auto BF = [](chq_mesh *m, int b, int d) { return b == 0 ? m->bf[0][d] : b < 3 ? m->sb[b][d] : m->bf[1][d]; };
     for (int b = 0; b < 4; ++b) {
       for (int j = 0; j < n; ++j) {
         chq_mesh *m = J[j];
@@ -1642,7 +1662,9 @@ int batch_build(chq_batch *B) {
         long nd = 0;
         c2[j] = c2p_args_ptr<P>(m, U(m, b), BF(m, b, 0), BF(m, b, 1), BF(m, b, 2), 0, nullptr, nullptr, skip);
         df[j] = diff_args<P>(m, BF(m, b, 0), BF(m, b, 1), BF(m, b, 2), skip, nd);
+        df[j].set = 1;
         rs[j] = res_emf_args<P>(m, BF(m, b, 0), BF(m, b, 1), BF(m, b, 2), skip, nullptr);
+        rs[j].set = 1;
       }
       o_sts_c2p[b] = push_vec(h, c2);
       o_sts_diff[b] = push_vec(h, df);
@@ -1663,6 +1685,8 @@ int batch_build(chq_batch *B) {
         a.mb1 = v ? m->smbj[0] : m->smb0[0]; a.mb2 = v ? m->smbj[1] : m->smb0[1]; a.mb3 = v ? m->smbj[2] : m->smb0[2];
         a.idx1 = 1.0 / g.dx1; a.idx2 = 1.0 / g.dx2; a.idx3 = 1.0 / g.dx3;
         a.done = B->sts_skip + j;
+        a.n0 = sts_first_component(m);
+        a.curl = m->cfg.eta > 0.0;
         dv[j] = a;
       }
       o_sts_div[v] = push_vec(h, dv);
@@ -1674,6 +1698,7 @@ int batch_build(chq_batch *B) {
         chq_mesh *m = J[j];
         StsCombArgs a{};
         a.g = m->g;
+        a.n0 = sts_first_component(m);
         a.out = U(m, form[v][0]); a.x = U(m, form[v][1]); a.y = U(m, form[v][2]); a.z = U(m, 0);
         a.p = v ? m->smj : m->sm0;
         a.q = m->sm0;
@@ -1688,11 +1713,11 @@ int batch_build(chq_batch *B) {
       }
       o_sts_comb[v] = push_vec(h, cb);
     }
-    std::vector<SpanArgs> zero(n), copy0(n);
-    for (int j = 0; j < n; ++j) {   // flux and EMF zero fill; Y0 = (u0, b?f0)
+    std::vector<SpanArgs> zero(n);   // flux and EMF zero fill
+    for (int j = 0; j < n; ++j) {
       chq_mesh *m = J[j];
       const long vs = (long)m->g.vstride;
-      SpanArgs z{}, c{};
+      SpanArgs z{};
       for (int d = 0; d < 3; ++d) {
         z.dst[d] = (unsigned long long *)m->flx[d];
         z.words[d] = NVAR * vs * (long)m->psize / 8;
@@ -1702,20 +1727,8 @@ int batch_build(chq_batch *B) {
       z.nspan = 6;
       z.done = B->sts_skip + j;
       zero[j] = z;
-      c.dst[0] = (unsigned long long *)m->sy[0];
-      c.src[0] = (const unsigned long long *)m->u[0];
-      c.words[0] = NVAR * vs;
-      for (int d = 0; d < 3; ++d) {
-        c.dst[1 + d] = (unsigned long long *)m->sb[0][d];
-        c.src[1 + d] = (const unsigned long long *)m->bf[0][d];
-        c.words[1 + d] = vs;
-      }
-      c.nspan = 4;
-      c.done = &m->ctl->done;
-      copy0[j] = c;
     }
     o_sts_zero = push_vec(h, zero);
-    o_sts_copy0 = push_vec(h, copy0);
   }
   const size_t o_status = h.push(std::vector<double>(3 * n + 1).data(), (3 * n + 1) * sizeof(double));
   // allocated and uploaded on the legacy default stream, which then completes both
@@ -1733,6 +1746,7 @@ int batch_build(chq_batch *B) {
   B->k_corner.slots = (BatchSlot *)(d + o_corner_s);
   B->k_update.slots = (BatchSlot *)(d + o_update_s);
   B->k_rerun.slots = (BatchSlot *)(d + o_rerun_s);
+  B->k_frame.slots = (BatchSlot *)(d + o_frame_s);
   B->k_flag.slots = (BatchSlot *)(d + o_flag_s);
   B->k_repair.slots = (BatchSlot *)(d + o_repair_s);
   B->k_limit.slots = (BatchSlot *)(d + o_limit_s);
@@ -1763,7 +1777,6 @@ int batch_build(chq_batch *B) {
     for (int v = 0; v < 2; ++v) B->a_sts_div[v] = d + o_sts_div[v];
     for (int v = 0; v < 5; ++v) B->a_sts_comb[v] = d + o_sts_comb[v];
     B->a_sts_zero = d + o_sts_zero;
-    B->a_sts_copy0 = d + o_sts_copy0;
   }
   for (int st = 0; st < B->nstage; ++st) {
     B->a_diff[st] = d + o_diff[st];
@@ -1874,17 +1887,18 @@ int batch_sts(chq_batch *B, cudaStream_t s, long long &L) {
   const double *coef_dev = reinterpret_cast<const double *>(B->sts_dyn + o_coef);
   const dim3 b2(32, 8);
   const unsigned nspan = (unsigned)B->k_span.nblocks;
-  pdl(span_batched, nspan, 256, 0, s, (const SpanArgs *)B->a_sts_copy0, B->k_span.slots, n);
-  CHQ_CUDA(cudaGetLastError());
-  ++L;
   for (int st = 1; st <= smax; ++st) {
     const int bi = wrote(st - 1), bo = wrote(st);
     const int form = st == 1 ? 0 : st == 2 ? 1 : 2 + (st % 3);
     pdl(sts_skip_kernel, (n + 127) / 128, 128, 0, s, B->sts_skip, nst_dev, n, st);
     pdl(c2p_batched<P>, (unsigned)B->k_c2p.nblocks, b2, 0, s, (const C2pArgs<P> *)B->a_sts_c2p[bi], B->k_c2p.slots, n);
-    pdl(span_batched, nspan, 256, 0, s, (const SpanArgs *)B->a_sts_zero, B->k_span.slots, n);
     CHQ_CUDA(cudaGetLastError());
-    L += 3;
+    L += 2;
+    if (std::find(nst.begin(), nst.end(), st) != nst.end()) {   // some member's last operator (sts_operator's clear)
+      pdl(span_batched, nspan, 256, 0, s, (const SpanArgs *)B->a_sts_zero, B->k_span.slots, n);
+      CHQ_CUDA(cudaGetLastError());
+      ++L;
+    }
     if (B->k_diff.nblocks) {
       pdl(diff_flux_batched<P>, (unsigned)B->k_diff.nblocks, 256, 0, s, (const DiffArgs<P> *)B->a_sts_diff[bi],
                                                                         B->k_diff.slots, n);
@@ -1895,10 +1909,10 @@ int batch_sts(chq_batch *B, cudaStream_t s, long long &L) {
                                                                          B->k_res.slots, n);
       ++L;
     }
-    pdl(sts_div_batched<P>, (unsigned)B->k_update.nblocks, b2, 0, s, (const StsDivArgs<P> *)B->a_sts_div[st == 1 ? 0 : 1],
-                                                                      B->k_update.slots, n);
-    pdl(sts_combine_batched, (unsigned)B->k_update.nblocks, b2, 0, s, (const StsCombArgs *)B->a_sts_comb[form],
-                                                                      B->k_update.slots, n,
+    pdl(sts_div_batched<P>, (unsigned)B->k_frame.nblocks, b2, 0, s, (const StsDivArgs<P> *)B->a_sts_div[st == 1 ? 0 : 1],
+                                                                      B->k_frame.slots, n);
+    pdl(sts_combine_batched, (unsigned)B->k_frame.nblocks, b2, 0, s, (const StsCombArgs *)B->a_sts_comb[form],
+                                                                      B->k_frame.slots, n,
                                                                       coef_dev + 5 * (size_t)(st - 1) * n);
     CHQ_CUDA(cudaGetLastError());
     L += 2;
