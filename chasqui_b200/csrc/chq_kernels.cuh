@@ -36,6 +36,17 @@ template <class P> CHQ_D P upwind(P flux, P left, P right) {
   return (flux > tol) ? left : (flux < -tol) ? right : P(0.5) * (left + right);
 }
 
+// E3 at the x3-edge (j-1/2, i-1/2) of plane point l
+template <class P> CHQ_D P corner_e3(const EmfArgs<P> &A, long l) {
+  const long sj = A.g.sj;
+  const P *c2 = A.ecc + 2 * A.g.vstride;
+  const P l2 = upwind(ldg(A.f1 + l - sj), ldg(A.e3x2 + l - 1) - ldg(c2 + l - sj - 1), ldg(A.e3x2 + l) - ldg(c2 + l - sj));
+  const P r2 = upwind(ldg(A.f1 + l), ldg(A.e3x2 + l - 1) - ldg(c2 + l - 1), ldg(A.e3x2 + l) - ldg(c2 + l));
+  const P l1 = upwind(ldg(A.f2 + l - 1), ldg(A.e3x1 + l - sj) - ldg(c2 + l - sj - 1), ldg(A.e3x1 + l) - ldg(c2 + l - 1));
+  const P r1 = upwind(ldg(A.f2 + l), ldg(A.e3x1 + l - sj) - ldg(c2 + l - sj), ldg(A.e3x1 + l) - ldg(c2 + l));
+  return P(0.25) * (((l2 + r2) + (l1 + r1)) + ((ldg(A.e3x2 + l - 1) + ldg(A.e3x2 + l)) + (ldg(A.e3x1 + l - sj) + ldg(A.e3x1 + l))));
+}
+
 // The edge EMFs stored at point (k, j, i): E1 at (k-1/2, j-1/2, i), E2 at (k-1/2, j, i-1/2),
 // E3 at (k, j-1/2, i-1/2), each where it is in range (src/physics.hpp:242-297).
 template <class P> CHQ_D void corner_point(const EmfArgs<P> &A, int k, int j, int i) {
@@ -46,7 +57,7 @@ template <class P> CHQ_D void corner_point(const EmfArgs<P> &A, int k, int j, in
   const long l = g.idx(k, j, i);
   if (g.three_d) {
     if (j > g.je + 1 || k > g.ke + 1) return;
-    const P *c0 = A.ecc, *c1 = A.ecc + vs, *c2 = A.ecc + 2 * vs;
+    const P *c0 = A.ecc, *c1 = A.ecc + vs;
     if (i <= g.ie) {   // E1 on x1-edges (k-1/2, j-1/2, i)
       const P l3 = upwind(ldg(A.f2 + l - sk), ldg(A.e1x3 + l - sj) - ldg(c0 + l - sk - sj), ldg(A.e1x3 + l) - ldg(c0 + l - sk));
       const P r3 = upwind(ldg(A.f2 + l), ldg(A.e1x3 + l - sj) - ldg(c0 + l - sj), ldg(A.e1x3 + l) - ldg(c0 + l));
@@ -61,13 +72,7 @@ template <class P> CHQ_D void corner_point(const EmfArgs<P> &A, int k, int j, in
       const P r1 = upwind(ldg(A.f3 + l), ldg(A.e2x1 + l - sk) - ldg(c1 + l - sk), ldg(A.e2x1 + l) - ldg(c1 + l));
       A.e2[l] = P(0.25) * (((l3 + r3) + (l1 + r1)) + ((ldg(A.e2x3 + l - 1) + ldg(A.e2x3 + l)) + (ldg(A.e2x1 + l - sk) + ldg(A.e2x1 + l))));
     }
-    if (k <= g.ke) {   // E3 on x3-edges (k, j-1/2, i-1/2)
-      const P l2 = upwind(ldg(A.f1 + l - sj), ldg(A.e3x2 + l - 1) - ldg(c2 + l - sj - 1), ldg(A.e3x2 + l) - ldg(c2 + l - sj));
-      const P r2 = upwind(ldg(A.f1 + l), ldg(A.e3x2 + l - 1) - ldg(c2 + l - 1), ldg(A.e3x2 + l) - ldg(c2 + l));
-      const P l1 = upwind(ldg(A.f2 + l - 1), ldg(A.e3x1 + l - sj) - ldg(c2 + l - sj - 1), ldg(A.e3x1 + l) - ldg(c2 + l - 1));
-      const P r1 = upwind(ldg(A.f2 + l), ldg(A.e3x1 + l - sj) - ldg(c2 + l - sj), ldg(A.e3x1 + l) - ldg(c2 + l));
-      A.e3[l] = P(0.25) * (((l2 + r2) + (l1 + r1)) + ((ldg(A.e3x2 + l - 1) + ldg(A.e3x2 + l)) + (ldg(A.e3x1 + l - sj) + ldg(A.e3x1 + l))));
-    }
+    if (k <= g.ke) A.e3[l] = corner_e3(A, l);   // E3 on x3-edges (k, j-1/2, i-1/2)
   } else {
     // 2D / 1D: E1 and E2 live on x3-edges that coincide with the x2- and x1-faces
     if (j > g.je + 1) return;
@@ -81,12 +86,7 @@ template <class P> CHQ_D void corner_point(const EmfArgs<P> &A, int k, int j, in
         A.e3[l + sj] = c;
       }
     } else {
-      const P *c2 = A.ecc + 2 * vs;
-      const P l2 = upwind(ldg(A.f1 + l - sj), ldg(A.e3x2 + l - 1) - ldg(c2 + l - sj - 1), ldg(A.e3x2 + l) - ldg(c2 + l - sj));
-      const P r2 = upwind(ldg(A.f1 + l), ldg(A.e3x2 + l - 1) - ldg(c2 + l - 1), ldg(A.e3x2 + l) - ldg(c2 + l));
-      const P l1 = upwind(ldg(A.f2 + l - 1), ldg(A.e3x1 + l - sj) - ldg(c2 + l - sj - 1), ldg(A.e3x1 + l) - ldg(c2 + l - 1));
-      const P r1 = upwind(ldg(A.f2 + l), ldg(A.e3x1 + l - sj) - ldg(c2 + l - sj), ldg(A.e3x1 + l) - ldg(c2 + l));
-      A.e3[l] = P(0.25) * (((l2 + r2) + (l1 + r1)) + ((ldg(A.e3x2 + l - 1) + ldg(A.e3x2 + l)) + (ldg(A.e3x1 + l - sj) + ldg(A.e3x1 + l))));
+      A.e3[l] = corner_e3(A, l);
     }
   }
 }
@@ -167,31 +167,46 @@ template <class P> struct UpdateArgs {
   int cap;                   // list capacity
 };
 
+// the edge EMFs of point l, from their arrays
+template <class P> struct StoredEmf {
+  const UpdateArgs<P> &A;
+  CHQ_D double e1(long l) const { return (double)ldg(A.e1 + l); }
+  CHQ_D double e2(long l) const { return (double)ldg(A.e2 + l); }
+  CHQ_D double e3(long l) const { return (double)ldg(A.e3 + l); }
+};
+// below 3-D: E1 and E2 are face EMFs and E3 is formed from the faces' (corner_point's values)
+template <class P> struct PlaneEmf {
+  const EmfArgs<P> &A;
+  CHQ_D double e1(long l) const { return (double)ldg(A.e1x2 + l); }
+  CHQ_D double e2(long l) const { return (double)ldg(A.e2x1 + l); }
+  CHQ_D double e3(long l) const { return (double)(A.g.two_d ? corner_e3(A, l) : ldg(A.e3x1 + l)); }
+};
+
 // new face fields; curl of the edge EMFs (src/physics.hpp:327-347)
-template <class P> CHQ_D double new_b1(const UpdateArgs<P> &A, long l, double g0, double g1, double bdt) {
+template <class P, class E> CHQ_D double new_b1(const UpdateArgs<P> &A, const E &em, long l, double g0, double g1, double bdt) {
   const Geom &g = A.g;
   double curl = 0.0;
-  if (g.two_d) curl += ((double)ldg(A.e3 + l + g.sj) - (double)ldg(A.e3 + l)) * A.idx2;
-  if (g.three_d) curl -= ((double)ldg(A.e2 + l + g.sk) - (double)ldg(A.e2 + l)) * A.idx3;
+  if (g.two_d) curl += (em.e3(l + g.sj) - em.e3(l)) * A.idx2;
+  if (g.three_d) curl -= (em.e2(l + g.sk) - em.e2(l)) * A.idx3;
   return g0 * A.b1a[l] + g1 * A.b1b[l] - bdt * curl;
 }
-template <class P> CHQ_D double new_b2(const UpdateArgs<P> &A, long l, double g0, double g1, double bdt) {
+template <class P, class E> CHQ_D double new_b2(const UpdateArgs<P> &A, const E &em, long l, double g0, double g1, double bdt) {
   const Geom &g = A.g;
-  double curl = -((double)ldg(A.e3 + l + 1) - (double)ldg(A.e3 + l)) * A.idx1;
-  if (g.three_d) curl += ((double)ldg(A.e1 + l + g.sk) - (double)ldg(A.e1 + l)) * A.idx3;
+  double curl = -(em.e3(l + 1) - em.e3(l)) * A.idx1;
+  if (g.three_d) curl += (em.e1(l + g.sk) - em.e1(l)) * A.idx3;
   return g0 * A.b2a[l] + g1 * A.b2b[l] - bdt * curl;
 }
-template <class P> CHQ_D double new_b3(const UpdateArgs<P> &A, long l, double g0, double g1, double bdt) {
+template <class P, class E> CHQ_D double new_b3(const UpdateArgs<P> &A, const E &em, long l, double g0, double g1, double bdt) {
   const Geom &g = A.g;
-  double curl = ((double)ldg(A.e2 + l + 1) - (double)ldg(A.e2 + l)) * A.idx1;
-  if (g.two_d) curl -= ((double)ldg(A.e1 + l + g.sj) - (double)ldg(A.e1 + l)) * A.idx2;
+  double curl = (em.e2(l + 1) - em.e2(l)) * A.idx1;
+  if (g.two_d) curl -= (em.e1(l + g.sj) - em.e1(l)) * A.idx2;
   return g0 * A.b3a[l] + g1 * A.b3b[l] - bdt * curl;
 }
 
 // GRAV: compile the gravity epilogue (a separate instantiation keeps the plain update's
 // register count, and with it its occupancy, unchanged)
 // The update of one point (k, j, i) of the face/edge frame, is <= i <= ie+1 (and so on).
-template <class P, bool GRAV = false> CHQ_D void update_point(const UpdateArgs<P> &A, int k, int j, int i, double bdt) {
+template <class P, bool GRAV, class E> CHQ_D void update_point(const UpdateArgs<P> &A, const E &em, int k, int j, int i, double bdt) {
   const Geom &g = A.g;
   const double g0 = A.g0, g1 = A.g1;
   const long l = g.idx(k, j, i);
@@ -229,9 +244,9 @@ template <class P, bool GRAV = false> CHQ_D void update_point(const UpdateArgs<P
     }
   }
   double nb1 = 0, nb2 = 0, nb3 = 0;
-  if (j <= g.je && k <= g.ke) nb1 = new_b1(A, l, g0, g1, bdt);
-  if (i <= g.ie && k <= g.ke && (g.two_d || j == g.js)) nb2 = new_b2(A, l, g0, g1, bdt);
-  if (i <= g.ie && j <= g.je && (g.three_d || k == g.ks)) nb3 = new_b3(A, l, g0, g1, bdt);
+  if (j <= g.je && k <= g.ke) nb1 = new_b1(A, em, l, g0, g1, bdt);
+  if (i <= g.ie && k <= g.ke && (g.two_d || j == g.js)) nb2 = new_b2(A, em, l, g0, g1, bdt);
+  if (i <= g.ie && j <= g.je && (g.three_d || k == g.ks)) nb3 = new_b3(A, em, l, g0, g1, bdt);
   if (cell) {
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) A.uout[n * vs + l] = un[n];
@@ -255,12 +270,31 @@ template <class P, bool GRAV = false> CHQ_D void update_body(const UpdateArgs<P>
   const int j = g.js + by * blockDim.y + threadIdx.y;
   const int k = g.ks + bz;
   if (i > g.ie + 1 || j > g.je + 1 || k > g.ke + 1) return;
-  update_point<P, GRAV>(A, k, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
+  update_point<P, GRAV>(A, StoredEmf<P>{A}, k, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
 }
 
 template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_kernel(const UpdateArgs<P> A) {
   pdl_begin();
   update_body<P, GRAV>(A, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// K2 and K3 in one launch below 3-D, where a stage of a small mesh is mostly launches: each
+// point stores its edge EMFs and forms again the two neighbouring E3 its face fields need.
+// OT 64^2 90.9 -> 86.8 us a cycle, 256^2 131 -> 127 us; planes of more than kPlaneUpdatePoints
+// keep the two launches (1000^2 mixed: 853 us a cycle apart, 856 us in one). In 3-D the three
+// EMFs of the neighbours cost more than the launch: a form that marched tiles up z and passed
+// them along took 2.4 ms where the two kernels take 1.5 at 256^3.
+constexpr long kPlaneUpdatePoints = 1L << 18;
+template <class P, bool GRAV>
+__global__ void __launch_bounds__(256) plane_update_kernel(const EmfArgs<P> E, const UpdateArgs<P> A) {
+  pdl_begin();
+  if (A.done && *A.done) return;
+  const Geom &g = A.g;
+  const int i = g.is + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int j = g.js + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  if (i > g.ie + 1 || j > g.je + 1) return;
+  corner_point<P>(E, g.ks, j, i);
+  update_point<P, GRAV>(A, PlaneEmf<P>{E}, g.ks, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
 }
 
 // FOFC re-run of the whole update: every point of the frame, blocks striding over its
@@ -270,7 +304,8 @@ template <class P, bool GRAV> CHQ_D void update_rerun_body(const UpdateArgs<P> &
   if (A.done && *A.done) return;
   if (*A.need <= A.need_min) return;
   const Geom &g = A.g;
-  const int nx = (g.ie + 2 - g.is + 31) / 32, ny = (g.je + 2 - g.js + 7) / 8, nz = g.ke + 2 - g.ks;
+  const int nx = (g.ie + 2 - g.is + 31) / 32, ny = (g.je + 2 - g.js + 7) / 8,
+            nz = g.three_d ? g.ke + 2 - g.ks : 1;   // update_grid
   const long tiles = (long)nx * ny * nz;
   for (long t = b; t < tiles; t += nb) {
     const long r = t / nx;
@@ -314,7 +349,7 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_reru
       const int j = jc + (p / 3) % rj - (rj >> 1);
       const int k = kc + p / (3 * rj) - (rk >> 1);
       if (i < g.is || i > g.ie + 1 || j < g.js || j > g.je + 1 || k < g.ks || k > g.ke + 1) continue;
-      update_point<P, GRAV>(A, k, j, i, bdt);
+      update_point<P, GRAV>(A, StoredEmf<P>{A}, k, j, i, bdt);
     }
   }
 }

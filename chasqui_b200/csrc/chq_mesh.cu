@@ -397,7 +397,7 @@ YzShape yz_shape(const chq_mesh *m, int d, int len) {
 // the least waves x (length + 0.6). Small meshes thus take one face a thread (OT 64^2: 22 us a
 // flux launch at length 4, the old rule's), large ones the longest march.
 int default_march(chq_mesh *const *ms, size_t n) {
-  const double resident = 148.0 * (ms[0]->mixed ? 6 : 3);   // y/z blocks of the PPM kernels (FluxYzMinBlocks)
+  const double resident = 148.0 * (ms[0]->mixed ? FluxYzMinBlocks<float>::v : FluxYzMinBlocks<double>::v);   // y/z blocks
   int best = 4;
   double least = 1e300;
   for (int L : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64}) {
@@ -575,7 +575,7 @@ UpdateArgs<P> update_args(chq_mesh *m, int out, double g0, double g1, double bdt
 
 Launch3 update_grid(const chq_mesh *m) {
   const Geom &g = m->g;
-  return plane_grid(g.ie + 2 - g.is, g.je + 2 - g.js, g.ke + 2 - g.ks);
+  return plane_grid(g.ie + 2 - g.is, g.je + 2 - g.js, g.three_d ? g.ke + 2 - g.ks : 1);
 }
 
 // the same frame with its upper plane below 3-D (the RKL2 kernels, which write faces there)
@@ -593,6 +593,19 @@ int do_update(chq_mesh *m, int out, double g0, double g1, double bdt, const doub
   if (a.grav.on) pdl(update_kernel<P, true>, L.grid, L.block, 0, s, a);
   else pdl(update_kernel<P, false>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
+  return CHQ_OK;
+}
+
+// corner EMFs and update of a 1-D or 2-D mesh in one launch
+template <class P>
+int do_plane_update(chq_mesh *m, int out, double g0, double g1, double bdt, const double *bdt_dev, const int *done,
+                    cudaStream_t s) {
+  const EmfArgs<P> e = corner_args<P>(m, done, nullptr);
+  const UpdateArgs<P> a = update_args<P>(m, out, g0, g1, bdt, bdt_dev, done, nullptr);
+  const Launch3 L = update_grid(m);
+  m->nlaunch += 1;
+  if (a.grav.on) CHQ_CUDA(pdl(plane_update_kernel<P, true>, L.grid, L.block, 0, s, e, a));
+  else CHQ_CUDA(pdl(plane_update_kernel<P, false>, L.grid, L.block, 0, s, e, a));
   return CHQ_OK;
 }
 
@@ -1013,15 +1026,18 @@ int run_stage_a(chq_mesh *m, int cur, int out, double g0, double g1, double bdt,
     Prof p(m, PK_LIMIT, s);
     if ((rc = DISPATCH_P(m, do_limit)(m, 7u, bdt, bdt_dev, &m->ctl->limiter_count, done, s))) return rc;
   }
-  {
-    Prof p(m, PK_CORNER, s);
-    if ((rc = DISPATCH_P(m, do_corner)(m, done, nullptr, s))) return rc;
-  }
-  if (dstage) {
-    Prof p(m, PK_DIFF, s);
-    if ((rc = DISPATCH_P(m, do_res_emf)(m, bc1, bc2, bc3, done, nullptr, s, 0))) return rc;
-  }
-  {
+  if (!m->g.three_d && !dstage && (long)m->g.nx1 * m->g.nx2 <= kPlaneUpdatePoints) {
+    Prof p(m, PK_UPDATE, s);
+    if ((rc = DISPATCH_P(m, do_plane_update)(m, out, g0, g1, bdt, bdt_dev, done, s))) return rc;
+  } else {
+    {
+      Prof p(m, PK_CORNER, s);
+      if ((rc = DISPATCH_P(m, do_corner)(m, done, nullptr, s))) return rc;
+    }
+    if (dstage) {
+      Prof p(m, PK_DIFF, s);
+      if ((rc = DISPATCH_P(m, do_res_emf)(m, bc1, bc2, bc3, done, nullptr, s, 0))) return rc;
+    }
     Prof p(m, PK_UPDATE, s);
     if ((rc = DISPATCH_P(m, do_update)(m, out, g0, g1, bdt, bdt_dev, done, s))) return rc;
   }
