@@ -425,8 +425,8 @@ CHQ_D void face_store(const DirView<P> &V, int lf, const P f[NFLX], P sl, P sr) 
   V.out[2][lf] = f[FMV];
   V.out[3][lf] = f[FMW];
   V.out[4][lf] = f[FEN];
-  // entropy flux upwinded with the mass flux, averaged at an exact zero
-  V.out[5][lf] = (f[FD] > P(0)) ? f[FD] * sl : (f[FD] < P(0)) ? f[FD] * sr : P(0.5) * (f[FD] * (sl + sr));
+  // entropy flux upwinded with the mass flux (the published mean at an exact zero is zero too)
+  V.out[5][lf] = f[FD] * ((f[FD] > P(0)) ? sl : sr);
   V.out[6][lf] = -f[FBY];
   V.out[7][lf] = f[FBZ];
 }

@@ -314,7 +314,7 @@ template <class T> CHQ_D T fast_speed_q(const MState<T> &s, T bn, T bsq, T gamma
   const T yd = rcp_a(s.d);
   const T a = quot(gp + bsq, s.d, yd);
   const T dd = s.d * s.d;
-  const T disc = a * a - quot(T(4) * gp * bn * bn, dd, yd * yd);
+  const T disc = fma_(T(-4), quot(gp * bn * bn, dd, yd * yd), a * a);   // the scaling by 4 is exact
   const T root = sqrt_q(disc);
   ok = ok && in_range(s.d) && in_range(a);
   return sqrt_q(T(0.5) * (a + (disc > RootFloor<T>::v ? root : T(0))));
@@ -340,7 +340,8 @@ CHQ_D void star_side_q(const MState<T> &S, T dm, T slm, T sms, T sm, T bn, T bns
                        bool &ok) {
   const T t = dm * sms;
   const T den = t - bnsq;
-  const bool deg = fabs_(den) <= T(1e-12) * (fabs_(t) + bnsq) + Tiny<T>::v;
+  // (star_side's tiny addend counts only where the products vanish, out of the quotients' range)
+  const bool deg = fabs_(den) <= T(1e-12) * (fabs_(t) + bnsq);
   const T y = rcp_a(den);
   const T nv = quot(bn * (sm - S.u), den, y);
   const T nb = quot(dm * slm - bnsq, den, y);
