@@ -1,0 +1,49 @@
+"""The update reads a register of zero weight through the other one: every pair of weights the
+integrators use and each output register, registers that differ, against the plain-C oracle
+(FP64, state and face fields bit for bit)."""
+import numpy as np
+import pytest
+
+from chasqui_b200 import Mesh, make_config
+
+WEIGHTS = [(1.0, 0.0, 1), (1.0, 0.0, 0), (0.0, 1.0, 1), (0.0, 1.0, 0), (0.75, 0.25, 1), (1.0 / 3.0, 2.0 / 3.0, 0)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(17, 13, 11), (33, 47, 1), (130, 1, 1)])
+def test_update_weights_equal_the_oracle(shape):
+    from oracle import portsim
+    mesh = Mesh(make_config(nx1=shape[0], nx2=shape[1], nx3=shape[2], cfl=0.3, tlim=10.0))
+    pc = portsim.port_cfg()
+    for k in ("nx1", "nx2", "nx3", "x1min", "x1max", "x2min", "x2max", "x3min", "x3max", "recon", "rsolver", "gamma",
+              "dfloor", "pfloor", "cfl", "de_eta", "lhlld_phi", "tlim", "dual_energy", "low_mach", "flatten",
+              "characteristic", "fofc", "flux_limiter", "cool_alpha"):
+        setattr(pc, k, getattr(mesh.cfg, k))
+    pc.ng, pc.nstage = mesh.ng, 3
+    port = portsim.PortSim(pc)
+    mesh.init_problem("blast", [10.0, 0.1, 0.2, 1.0, 30.0, 1e-2, 11])
+    for f in ("u0", "b1f0", "b2f0", "b3f0"):
+        port.set(f, mesh.get(f))
+    mesh.prime(0.0)
+    port.prime(0.0)
+    mesh.fluxes_all(0)
+    mesh.corner_emf()
+    for d in range(1 + mesh.two_d + mesh.three_d):
+        portsim.lib().port_fluxes(port._h, d, 0)
+    portsim.lib().port_corner_emf(port._h)
+    rng = np.random.default_rng(3)
+    regs = {f + "%d" % r: rng.normal(size=mesh.shape(f + "%d" % r)) for f in ("u", "b1f", "b2f", "b3f") for r in (0, 1)}
+    bad = {}
+    for g0, g1, out in WEIGHTS:
+        for f, a in regs.items():
+            mesh.set(f, a)
+            port.set(f, a)
+        mesh.update(out, g0, g1, 1e-3)
+        portsim.lib().port_update(port._h, out, g0, g1, 1e-3)
+        for f in ("u%d", "b1f%d", "b2f%d", "b3f%d"):
+            got, want = mesh.get(f % out).ravel(), port.get(f % out)
+            if not np.array_equal(got, want):
+                bad[(g0, g1, out, f)] = (int((got != want).sum()), float(np.abs(got - want).max()))
+    port.close()
+    mesh.close()
+    assert not bad, bad
