@@ -329,12 +329,13 @@ template <int RE, class P> struct WindowStencil {
 // ---------------------------------------------------------------------------------------
 // Face work: Riemann solve of the face `lf` (between cells lf - stride and lf).
 //
-// What bounds it: FP64 issue (61 % of the FP64 pipe's cycles in the y/z launch, 71 % in the x
-// launch at 128^3). With compiled divisions and branching limiters a face took 2200 warp
-// instructions at 24 of 32 active lanes and waited on instruction fetch; with chq_quot.cuh and
-// selects it takes 1760, and the FP64 PPM + HLLD flux launch went from 0.880 to 0.539 ms at
-// 128^3 (blast), 5.21 to 3.54 ms at 256^3 (mixed: 2.88 to 2.09 ms), WENO-Z from 1.92 to 0.96 ms
-// at 128^3, OT 256^2 from 43 to 22 us.
+// What bounds it: FP64 issue (61 % of the FP64 pipe's cycles in the y/z launch, 68 % in the x
+// launch at 128^3; 730 FP64 operations a face and thread). With compiled divisions and branching
+// limiters a face took 2200 warp instructions at 24 of 32 active lanes and waited on instruction
+// fetch; with chq_quot.cuh and selects it takes 1380 at 31.6, and the FP64 PPM + HLLD flux launch
+// went from 0.880 to 0.444 ms at 128^3 (blast), 5.21 to 3.20 ms at 256^3 (mixed: 2.89 to 1.85 ms),
+// WENO-Z from 1.92 to 0.78 ms at 128^3, OT 256^2 from 43 to 16 us (rows laid end to end and
+// balanced marches included).
 
 // low-Mach blend of the normal velocities, Thornber et al. (2008) (src/physics.hpp:170-178)
 template <class P> CHQ_D void low_mach_blend(MState<P> &L, MState<P> &R, P cl, P cr) {
