@@ -12,9 +12,11 @@
 //   quot(a, b, y)   RN(a/b) for y = rcp_a(b): Markstein's correction of q = RN(a y) by the
 //                   exact remainder. The corrected value differs from a/b by less than
 //                   2^-51 ulp before its rounding, so it can miss RN(a/b) only when a/b lies
-//                   that close to a rounding midpoint (FP32, whose seed is used as it
-//                   is: 2^-20 ulp, about one result in 10^5 one unit off). The remainder is formed as b q - a and
-//                   subtracted, which keeps the sign of a zero numerator for b > 0.
+//                   that close to a rounding midpoint. FP32 uses the hardware seed as it
+//                   is (one unit at most): every reciprocal's correction, every root and 2^30
+//                   quotients over all significands of the divisor came out IEEE on a B200.
+//                   The remainder is formed as b q - a and subtracted, which keeps the sign of
+//                   a zero numerator for b > 0.
 //   sqrt_q(x, ih)   RN(sqrt x) by Goldschmidt's iteration from the reciprocal-square-root seed
 //                   with a third-order step and Markstein's final correction (as accurate as
 //                   quot); ih receives 1 / sqrt(x) to about an ulp, so that a quotient by the
@@ -24,7 +26,8 @@
 // Valid for finite numerators and for divisors and radicands that in_range accepts (FP64
 // 2^-300 .. 2^300, FP32 2^-36 .. 2^60, positive); outside it the caller takes the plain
 // operations. Compiles for the host with the seeds emulated at their documented 20 (FP64) and
-// 22 (FP32) bits (tests/quot_check.cpp compares every function with the IEEE operation).
+// 22 (FP32) bits (tests/quot_check.cpp compares every function with the IEEE operation; with
+// the coarser FP32 seed one quotient in 10^5 is one unit off there).
 #pragma once
 #include "chq_divide.cuh"
 #include <cmath>
@@ -128,6 +131,12 @@ template <class T> CHQ_DIV_HD T sqrt_q(T x) {
   T ih;
   return sqrt_q(x, ih);
 }
+
+// a b + c in the form's own arithmetic: two roundings in FP64, one in FP32 (the mixed form lets
+// products contract). Written out where a product is shared by several sums, which the compiler
+// would otherwise round once for all of them.
+CHQ_DIV_HD double mad(double a, double b, double c) { return a * b + c; }
+CHQ_DIV_HD float mad(float a, float b, float c) { return fma_(a, b, c); }
 
 // radicands below this are negligible beside any in_range value they are added to the root of
 // (their root is at most 2^-150 resp. 2^-24 of it) and count as zero

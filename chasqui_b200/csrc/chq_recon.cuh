@@ -24,7 +24,9 @@ template <class T> CHQ_D T vl_slope(T qm, T q0, T qp) {
 // The pieces below are written without branches: a warp's cells differ in which limiter
 // applies, and a branch costs its lanes both sides. Scaling by a power of two is exact, so
 // factors of 2, 1/2 and 1/4 are moved to where they cost nothing; every rounded operation has
-// the published operands.
+// the published operands. In FP32 a product and the sum it enters round once (mad), also where
+// the product is shared: with 3 q and 11 q, 5 q, 3 q of WENO-Z rounded first, the error of the
+// FP32 face fluxes against FP64 was 1 to 7 % (PPM) and up to 0.6 % (WENO-Z) larger on smooth states.
 
 // twice the monotonised central slope, CW84 eq. 1.8 (src/recon.hpp:21-27):
 // sgn(dc) min(|dc|, 2 min(|dl|, |dr|)) with dc = (qp - qm)/2, zero at an extremum
@@ -48,9 +50,9 @@ template <class T> CHQ_HD void ppm_limit(T q, T &qL, T &qR) {
   const bool flat = (r - q) * (q - l) <= T(0);
   const T d = r - l;
   const T c = fma_(T(-0.5), l + r, q);
-  const T t = sixth(d * d), dc = d * c, q3 = T(3) * q;
-  const T nl = (dc > t) ? fma_(T(-2), r, q3) : l;
-  const T nr = (dc < -t) ? fma_(T(-2), l, q3) : r;
+  const T t = sixth(d * d), dc = d * c;
+  const T nl = (dc > t) ? mad(T(3), q, T(-2) * r) : l;
+  const T nr = (dc < -t) ? mad(T(3), q, T(-2) * l) : r;
   qL = flat ? q : nl;
   qR = flat ? q : nr;
 }
@@ -107,12 +109,18 @@ template <class T> struct WenoLimit;   // indicators and weights above this: pla
 template <> struct WenoLimit<double> { static constexpr double v = 0x1p+300; };
 template <> struct WenoLimit<float> { static constexpr float v = 0x1p+96f; };
 
+// six times the substencils' values at the face above the middle cell (the outer, the middle
+// and the inner one, cells in order towards the face)
+template <class T> CHQ_HD T weno_outer(T a, T b, T c) { return mad(T(11), c, mad(T(-7), b, T(2) * a)); }
+template <class T> CHQ_HD T weno_mid(T a, T b, T c) { return fma_(T(2), c, mad(T(5), b, -a)); }
+template <class T> CHQ_HD T weno_inner(T a, T b, T c) { return mad(T(5), b, T(2) * a) - c; }
+
 template <bool PLAIN, class T> CHQ_D bool wenoz_both(const T q[5], T &aL, T &aR) {
   const T eps = Tiny<T>::weno_eps;
   const T c13 = T(13) / T(12);
-  const T b0 = c13 * sqr(fma_(T(-2), q[1], q[0] + q[2])) + T(0.25) * sqr(fma_(T(-4), q[1], T(3) * q[2] + q[0]));
+  const T b0 = c13 * sqr(fma_(T(-2), q[1], q[0] + q[2])) + T(0.25) * sqr(fma_(T(-4), q[1], mad(T(3), q[2], q[0])));
   const T b1 = c13 * sqr(fma_(T(-2), q[2], q[1] + q[3])) + T(0.25) * sqr(q[1] - q[3]);
-  const T b2 = c13 * sqr(fma_(T(-2), q[3], q[4] + q[2])) + T(0.25) * sqr(fma_(T(-4), q[3], T(3) * q[2] + q[4]));
+  const T b2 = c13 * sqr(fma_(T(-2), q[3], q[4] + q[2])) + T(0.25) * sqr(fma_(T(-4), q[3], mad(T(3), q[2], q[4])));
   const T tau = fabs_(b0 - b2);
   auto ratio = [&](T b) { return PLAIN ? tau / b : quot(tau, b, rcp_a(b)); };
   const T d0 = T(1) + ratio(b0 + eps), d1 = T(1) + ratio(b1 + eps), d2 = T(1) + ratio(b2 + eps);
@@ -120,11 +128,10 @@ template <bool PLAIN, class T> CHQ_D bool wenoz_both(const T q[5], T &aL, T &aR)
   const T l0 = T(0.1) * d2, l2 = T(0.3) * d0, r0 = T(0.1) * d0, r2 = T(0.3) * d2;
   const T sr = r0 + a1 + r2, sl = l0 + a1 + l2;
   const T ir = PLAIN ? T(1) / sr : rcp_rn(sr), il = PLAIN ? T(1) / sl : rcp_rn(sl);
-  const T q11 = T(11) * q[2], q5 = T(5) * q[2], q2 = T(2) * q[2];
-  aR = ir * (r0 * sixth(T(2) * q[0] - T(7) * q[1] + q11) + a1 * sixth(fma_(T(2), q[3], -q[1] + q5)) +
-             r2 * sixth(q2 + T(5) * q[3] - q[4]));
-  aL = il * (l0 * sixth(T(2) * q[4] - T(7) * q[3] + q11) + a1 * sixth(fma_(T(2), q[1], -q[3] + q5)) +
-             l2 * sixth(q2 + T(5) * q[1] - q[0]));
+  aR = ir * (r0 * sixth(weno_outer(q[0], q[1], q[2])) + a1 * sixth(weno_mid(q[1], q[2], q[3])) +
+             r2 * sixth(weno_inner(q[2], q[3], q[4])));
+  aL = il * (l0 * sixth(weno_outer(q[4], q[3], q[2])) + a1 * sixth(weno_mid(q[3], q[2], q[1])) +
+             l2 * sixth(weno_inner(q[2], q[1], q[0])));
   return sr < WenoLimit<T>::v && sl < WenoLimit<T>::v && (b0 + b1) + b2 < WenoLimit<T>::v;
 }
 template <class T> __device__ __noinline__ void wenoz_plain(T *v) {
