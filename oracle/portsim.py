@@ -83,6 +83,21 @@ def cfg_from_chq(c: dict) -> port_cfg:
     return p
 
 
+def of_mesh(mesh, nstage=3) -> "PortSim":
+    """a PortSim of a device mesh's configuration (bc, gravity and cooling coefficients included)"""
+    p = port_cfg()
+    c = mesh.cfg
+    for k in ("nx1", "nx2", "nx3", "x1min", "x1max", "x2min", "x2max", "x3min", "x3max", "recon", "rsolver", "gamma",
+              "dfloor", "pfloor", "cfl", "de_eta", "lhlld_phi", "tlim", "dual_energy", "low_mach", "flatten",
+              "characteristic", "fofc", "flux_limiter", "cool_alpha", "nu", "kappa", "eta", "sts", "g1", "g2", "g3",
+              "gm", "gx0", "gy0", "gz0", "rsoft", "cooling", "lambda0", "tfloor"):
+        setattr(p, k, getattr(c, k))
+    p.grav_uniform, p.grav_point = c.gravity_uniform, c.gravity_point
+    p.bc[0], p.bc[1], p.bc[2] = c.bc1, c.bc2, c.bc3
+    p.ng, p.nstage = mesh.ng, nstage
+    return PortSim(p)
+
+
 class PortSim:
     def __init__(self, cfg: port_cfg):
         self._h = lib().port_create(C.byref(cfg))

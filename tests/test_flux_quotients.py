@@ -53,13 +53,7 @@ def test_fluxes_equal_the_oracle(shape, scheme):
     low = int(scheme.endswith("lowmach"))
     cfg = dict(nx1=n1, nx2=n2, nx3=n3, recon=recon, rsolver=solver, characteristic=char, low_mach=low)
     mesh = Mesh(make_config(**cfg))
-    pc = portsim.port_cfg()
-    for k in ("nx1", "nx2", "nx3", "x1min", "x1max", "x2min", "x2max", "x3min", "x3max", "recon", "rsolver", "gamma",
-              "dfloor", "pfloor", "cfl", "de_eta", "lhlld_phi", "tlim", "dual_energy", "low_mach", "flatten",
-              "characteristic", "fofc", "flux_limiter", "cool_alpha"):
-        setattr(pc, k, getattr(mesh.cfg, k))
-    pc.ng, pc.nstage = mesh.ng, 3
-    port = portsim.PortSim(pc)
+    port = portsim.of_mesh(mesh)
     rng = np.random.default_rng(7)
     cells, faces = mesh.shape("w")[1:], mesh.shape("b1f0")[1:]
     dirs = [0] + [1] * mesh.two_d + [2] * mesh.three_d

@@ -17,13 +17,7 @@ def test_cycles_below_3d_equal_the_oracle(name):
     from oracle import portsim
     n1, n2, n3, cycles = SHAPES[name]
     mesh = Mesh(make_config(nx1=n1, nx2=n2, nx3=n3, x1min=-.5, x1max=.5, x2min=-.5, x2max=.5, cfl=0.4, tlim=10.0))
-    pc = portsim.port_cfg()
-    for k in ("nx1", "nx2", "nx3", "x1min", "x1max", "x2min", "x2max", "x3min", "x3max", "recon", "rsolver", "gamma",
-              "dfloor", "pfloor", "cfl", "de_eta", "lhlld_phi", "tlim", "dual_energy", "low_mach", "flatten",
-              "characteristic", "fofc", "flux_limiter", "cool_alpha"):
-        setattr(pc, k, getattr(mesh.cfg, k))
-    pc.ng, pc.nstage = mesh.ng, 3
-    port = portsim.PortSim(pc)
+    port = portsim.of_mesh(mesh)
     mesh.init_problem("blast", [1e4, 1e-3, 0.2, 1.0, 30.0, 1e-2, 11])   # strong enough for FOFC repairs
     for f in ("u0", "b1f0", "b2f0", "b3f0"):
         port.set(f, mesh.get(f))

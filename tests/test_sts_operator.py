@@ -20,13 +20,7 @@ def test_rkl2_cycles_equal_the_oracle(shape, coef):
     n1, n2, n3 = SHAPES[shape]
     nu, kappa, eta = COEF[coef]
     mesh = Mesh(make_config(nx1=n1, nx2=n2, nx3=n3, nu=nu, kappa=kappa, eta=eta, sts=1, tlim=10.0))
-    pc = portsim.port_cfg()
-    for k in ("nx1", "nx2", "nx3", "x1min", "x1max", "x2min", "x2max", "x3min", "x3max", "recon", "rsolver", "gamma",
-              "dfloor", "pfloor", "cfl", "de_eta", "lhlld_phi", "tlim", "dual_energy", "low_mach", "flatten",
-              "characteristic", "fofc", "flux_limiter", "cool_alpha", "nu", "kappa", "eta", "sts"):
-        setattr(pc, k, getattr(mesh.cfg, k))
-    pc.ng, pc.nstage = mesh.ng, 3
-    port = portsim.PortSim(pc)
+    port = portsim.of_mesh(mesh)
     mesh.init_problem("orszag_tang" if n3 == 1 else "cpaw", [2.0] if n3 == 1 else [1, 1, 1, 1.0, 0.3, 1.0, 0.2])
     for f in ("u0", "b1f0", "b2f0", "b3f0"):
         port.set(f, mesh.get(f))

@@ -14,13 +14,7 @@ WEIGHTS = [(1.0, 0.0, 1), (1.0, 0.0, 0), (0.0, 1.0, 1), (0.0, 1.0, 0), (0.75, 0.
 def test_update_weights_equal_the_oracle(shape):
     from oracle import portsim
     mesh = Mesh(make_config(nx1=shape[0], nx2=shape[1], nx3=shape[2], cfl=0.3, tlim=10.0))
-    pc = portsim.port_cfg()
-    for k in ("nx1", "nx2", "nx3", "x1min", "x1max", "x2min", "x2max", "x3min", "x3max", "recon", "rsolver", "gamma",
-              "dfloor", "pfloor", "cfl", "de_eta", "lhlld_phi", "tlim", "dual_energy", "low_mach", "flatten",
-              "characteristic", "fofc", "flux_limiter", "cool_alpha"):
-        setattr(pc, k, getattr(mesh.cfg, k))
-    pc.ng, pc.nstage = mesh.ng, 3
-    port = portsim.PortSim(pc)
+    port = portsim.of_mesh(mesh)
     mesh.init_problem("blast", [10.0, 0.1, 0.2, 1.0, 30.0, 1e-2, 11])
     for f in ("u0", "b1f0", "b2f0", "b3f0"):
         port.set(f, mesh.get(f))
