@@ -404,8 +404,8 @@ CHQ_D bool face_solve(const FluxArgs<P> &A, const DirView<P> &V, int lf, const P
       chi = divz(fmax_(flow_speed_u(L, b_n), flow_speed_u(R, b_n)), cfmax);
     } else {
       ok = ok && in_range(den) && in_range(cfmax);
-      ratio = quot(num, den, rcp_a(den));
-      chi = quot(fmax_(flow_speed_q(L, b_n), flow_speed_q(R, b_n)), cfmax, rcp_a(cfmax));
+      ratio = quot(num, den, rcp_n(den));
+      chi = quot(fmax_(flow_speed_q(L, b_n), flow_speed_q(R, b_n)), cfmax, rcp_n(cfmax));
     }
     ratio = fmin_(P(1), ratio);
     chi = fmin_(P(1), chi);

@@ -430,7 +430,7 @@ CHQ_D void fofc_flag_body(const FlagArgs &A, int bx, int by, int bz) {
     const double d = A.u[IDN * vs + l], m1 = A.u[IM1 * vs + l], m2 = A.u[IM2 * vs + l], m3 = A.u[IM3 * vs + l];
     const double en = A.u[IEN * vs + l];
     const double mm = 0.5 * (sqr(m1) + sqr(m2) + sqr(m3));
-    const double ke = in_range(d) ? quot(mm, d, rcp_a(d)) : divz(mm, d);
+    const double ke = in_range(d) ? quot(mm, d, rcp_n(d)) : divz(mm, d);
     const double eint = en - ke - 0.5 * (bx * bx + by * by + bz * bz);
     double p = A.eos.gm1 * eint;
     if (A.eos.dual_energy && eint < A.eos.de_eta * fabs(en)) p = (A.u[IENT * vs + l] / d) * pow(d, A.eos.gamma);
@@ -939,7 +939,7 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
     } else {
       p = fmax(p, e.pfloor);
       const double dg = pow(d, e.gamma);
-      sent = in_range(dg) ? quot(p, dg, rcp_a(dg)) : p / dg;
+      sent = in_range(dg) ? quot(p, dg, rcp_n(dg)) : p / dg;
       A.u[IENT * vs + l] = d * sent;
     }
     A.w[IDN * vs + l] = P(d);
@@ -963,7 +963,7 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
         if (ok) {
           const double root = sqrt_q(disc);
           const double s = fabs(v) + sqrt_q(0.5 * (a + (disc > RootFloor<double>::v ? root : 0.0)));
-          if (in_range(s)) return quot(dx, s, rcp_a(s));
+          if (in_range(s)) return quot(dx, s, rcp_n(s));
         }
         return dx / (fabs(v) + sqrt(0.5 * (a + sqrt(fmax(disc, 0.0)))));
       };

@@ -311,7 +311,7 @@ CHQ_HD void hlld(const MState<T> &L, const MState<T> &R, T bn, T gamma, T gm1, T
 // fast magnetosonic speed (fast_speed) from bsq = B^2
 template <class T> CHQ_D T fast_speed_q(const MState<T> &s, T bn, T bsq, T gamma, bool &ok) {
   const T gp = gamma * s.p;
-  const T yd = rcp_a(s.d);
+  const T yd = rcp_n(s.d);
   const T a = quot(gp + bsq, s.d, yd);
   const T dd = s.d * s.d;
   const T disc = fma_(T(-4), quot(gp * bn * bn, dd, yd * yd), a * a);   // the scaling by 4 is exact
@@ -323,7 +323,7 @@ template <class T> CHQ_D T fast_speed_q(const MState<T> &s, T bn, T bsq, T gamma
 // modified fast speed of LHLLD (flow_speed_u)
 template <class T> CHQ_D T flow_speed_q(const MState<T> &s, T bn) {
   const T vsq = s.u * s.u + s.v * s.v + s.w * s.w;
-  const T yd = rcp_a(s.d);
+  const T yd = rcp_n(s.d);
   const T casq = quot(bn * bn + s.by * s.by + s.bz * s.bz, s.d, yd);
   const T caxsq = quot(bn * bn, s.d, yd);
   const T a = casq + vsq;
@@ -342,7 +342,7 @@ CHQ_D void star_side_q(const MState<T> &S, T dm, T slm, T sms, T sm, T bn, T bns
   const T den = t - bnsq;
   // (star_side's tiny addend counts only where the products vanish, out of the quotients' range)
   const bool deg = fabs_(den) <= T(1e-12) * (fabs_(t) + bnsq);
-  const T y = rcp_a(den);
+  const T y = rcp_n(den);
   const T nv = quot(bn * (sm - S.u), den, y);
   const T nb = quot(dm * slm - bnsq, den, y);
   vs = deg ? S.v : S.v - S.by * nv;
@@ -429,14 +429,14 @@ CHQ_D bool hlld_q(const MState<T> &L, const MState<T> &R, T bn, T gm1, T rgm1, T
   const T pts = ((dsr * ptl - dsl * ptr) + (phi * ((L.d * R.d) * (srmr * slml))) * (R.u - L.u)) * iden;
   // left divisors negated (S_M - S_L > 0), which negates the numerators: the same quotients
   const T nl = sm - sl, nr = sr - sm;
-  const T yl = rcp_a(nl), yr = rcp_a(nr);
+  const T yl = rcp_n(nl), yr = rcp_n(nr);
   const T dls = quot(-dsl, nl, yl), drs = quot(dsr, nr, yr);
   bool ok = in_range(dds) && in_range(nl) && in_range(nr) && in_range(dls) && in_range(drs);
   T yql, yqr;
   const T sqdl = sqrt_q(dls, yql), sqdr = sqrt_q(drs, yqr);
   const T abn = fabs_(bn);
-  const T sls = sm - quot(abn, sqdl, yql);
-  const T srs = sm + quot(abn, sqdr, yqr);
+  const T sls = sm - quot(abn, sqdl, rcp_root(sqdl, yql));
+  const T srs = sm + quot(abn, sqdr, rcp_root(sqdr, yqr));
   // region and side as in hlld
   const bool star_l = sls > T(0);
   const bool star_r = !star_l && (srs < T(0));

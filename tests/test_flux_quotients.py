@@ -1,8 +1,9 @@
 """The face-flux kernels' branch-free solver against the plain-C oracle, bit for bit (FP64), on
 states that reach each of its paths: ordinary shocks, gas at rest (both sides averaged), no
 field (single-star region), supersonic flow, and states whose divisors leave the range of the
-shared reciprocals, where the face is solved again with plain divisions. One NaN cell must
-spread to the same faces. Ragged extents leave partial warps, tiles and march segments."""
+shared reciprocals, where the face is solved again with plain divisions, and a gas whose density,
+sound speed and field are a few units from 1, where quotients lie closest to rounding midpoints. One
+NaN cell must spread to the same faces. Ragged extents leave partial warps, tiles and march segments."""
 import numpy as np
 import pytest
 
@@ -11,7 +12,7 @@ from chasqui_b200 import Mesh, make_config
 SHAPES = {"3d": (37, 9, 7), "2d": (66, 35, 1), "1d": (130, 1, 1)}
 SCHEMES = {"plm_hlld": (1, 1, 0), "ppm_hlld": (2, 1, 0), "wenoz_hlld": (3, 1, 0), "ppmx_lhlld": (4, 2, 0),
            "ppm_lhlld": (2, 2, 0), "ppm_hlld_char": (2, 1, 1), "wenoz_hlld_lowmach": (3, 1, 0)}
-KINDS = ("random", "rest", "rest_noise", "no_field", "supersonic", "stiff", "out_of_range", "nan")
+KINDS = ("random", "rest", "rest_noise", "no_field", "supersonic", "stiff", "out_of_range", "nan", "near_one")
 
 
 def states(kind, shp, rng):
@@ -37,6 +38,11 @@ def states(kind, shp, rng):
         far = rng.random(shp) < 0.2
         p = np.where(far, 1e120, p)
         d = np.where(rng.random(shp) < 0.1, 1e-9, d)
+    if kind == "near_one":
+        def near(a):
+            return a + rng.integers(-4, 3, shp) * 2.0 ** -53
+        d, p = near(1.0), near(0.6)
+        v, b = [rng.integers(-2, 3, shp) * 2.0 ** -50 for _ in range(3)], [near(1.0), near(0.0), near(0.0)]
     w = np.stack([d, v[0], v[1], v[2], p, p / d ** (5.0 / 3.0)])
     if kind == "nan":
         w[1, shp[0] // 2, shp[1] // 2, shp[2] // 2] = np.nan
@@ -78,3 +84,27 @@ def test_fluxes_equal_the_oracle(shape, scheme):
     port.close()
     mesh.close()
     assert not bad, bad
+
+
+@pytest.mark.gpu
+def test_cons_to_prim_next_to_one_equals_the_oracle():
+    """densities (and, at rest, sound speeds) a few units from 1: velocities and the time step bit for bit"""
+    from oracle import portsim
+    mesh = Mesh(make_config(nx1=64, nx2=64, nx3=1, cfl=0.4))
+    port = portsim.of_mesh(mesh)
+    rng = np.random.default_rng(5)
+    shp = mesh.shape("u0")
+    u = np.zeros(shp)
+    u[0] = 1.0 + rng.integers(-4, 3, shp[1:]) * 2.0 ** -53
+    u[1:4] = rng.choice([0.0, 1.0, 0.5, 0.75], (3,) + shp[1:])
+    u[4] = 0.9 + 0.5 * (u[1:4] ** 2).sum(0) / u[0]   # gamma p = 1
+    for s in (mesh, port):
+        s.set("u0", u)
+        for q in (1, 2, 3):
+            s.set("b%df0" % q, np.zeros(mesh.shape("b1f0")))
+    dt, want = mesh.cons_to_prim(0, True), portsim.lib().port_cons_to_prim(port._h, 0, 1)
+    got, exp = mesh.get("w"), port.get("w").reshape(mesh.shape("w"))
+    port.close()
+    mesh.close()
+    assert dt == want
+    assert np.array_equal(got[:5], exp[:5]), [int((got[n] != exp[n]).sum()) for n in range(5)]
