@@ -127,9 +127,8 @@ CHQ_D void batch_block(const BatchSlot &sl, long b, int &bx, int &by, int &bz) {
 // OT 64^2 132 -> 122 us a cycle, 256^2 177 -> 162 us. Larger grids lose by it (256^3 FP64 19.0
 // -> 19.2 ms, mixed 13.7 -> 14.0 ms a cycle): their waiting blocks take the place of running ones.
 constexpr unsigned long long kPdlBlocks = 148 * 10;
-CHQ_D void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 CHQ_D void pdl_begin() {
-  pdl_wait();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 

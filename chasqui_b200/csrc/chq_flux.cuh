@@ -844,16 +844,15 @@ template <int R, class P> __host__ __device__ constexpr size_t flux_yz_smem() {
 
 template <int R, int S, bool CHAR, class P, int V = 0>
 __global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_kernel(const __grid_constant__ FluxArgs<P> A) {
-  // The x sweep reads and writes nothing of the y/z launch before it, whose blocks have all
-  // passed their own wait when this one starts: it runs beside the y/z launch's last wave and
-  // waits for it at the end, so that it completes last. Alone it waits first.
-  if (A.nblk[1] + A.nblk[2] == 0) pdl_wait();
+  // (it shares no data with the y/z launch, but reads what con2prim wrote before that: only its
+  // own wait makes those writes visible to it)
+  pdl_begin();
+  if (A.skip && *A.skip) return;
   const int wid = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 5);
-  if (!(A.skip && *A.skip) && wid < A.nxwarp) {
+  if (wid < A.nxwarp) {
     if constexpr (R == R_PPM && !CHAR) sweep_x_ppm<S, P>(A, wid);
     else sweep_x<R, S, CHAR, P>(A, wid);
   }
-  pdl_wait();
 }
 
 template <int R, int S, bool CHAR, class P>
@@ -896,17 +895,17 @@ __global__ void __launch_bounds__(kYzThreads, FluxYzMinBlocks<double>::v)
 // batched forms: the blocks of many meshes in one launch per sweep kind (chq_batch); each
 // block copies its mesh's arguments to shared memory first
 template <int R, int S, bool CHAR, class P, int V = 0>
-__global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_batched(const FluxArgs<P> *args, const BatchSlot *slots, int n, int alone) {
-  if (alone) pdl_wait();   // as in flux_x_kernel: no y/z launch before this one
+__global__ void __launch_bounds__(128, (FluxMinBlocks<P, V>::v)) flux_x_batched(const FluxArgs<P> *args, const BatchSlot *slots, int n) {
+  pdl_begin();
   __shared__ __align__(16) unsigned char sa[sizeof(FluxArgs<P>)];
   const int j = batch_job(slots, n, blockIdx.x);
   const FluxArgs<P> &A = stage_args(args, j, sa);
+  if (A.skip && *A.skip) return;
   const int wid = (int)(blockIdx.x - slots[j].off) * 4 + (int)(threadIdx.x >> 5);
-  if (!(A.skip && *A.skip) && wid < A.nxwarp) {
+  if (wid < A.nxwarp) {
     if constexpr (R == R_PPM && !CHAR) sweep_x_ppm<S, P>(A, wid);
     else sweep_x<R, S, CHAR, P>(A, wid);
   }
-  pdl_wait();
 }
 
 template <int R, class P> __host__ __device__ constexpr size_t flux_yz_batched_smem() {

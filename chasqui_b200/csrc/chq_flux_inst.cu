@@ -86,8 +86,8 @@ static cudaError_t gob(const FluxArgs<CHQ_P> *a, const BatchSlot *sx, const Batc
     if (e2 != cudaSuccess) return e2;
   }
   if (nbx) {
-    if (xvar) pdl(flux_x_batched<CHQ_R, S, C, CHQ_P, 1>, nbx, 128, 0, s, a, sx, n, nbyz == 0);
-    else pdl(flux_x_batched<CHQ_R, S, C, CHQ_P, 0>, nbx, 128, 0, s, a, sx, n, nbyz == 0);
+    if (xvar) pdl(flux_x_batched<CHQ_R, S, C, CHQ_P, 1>, nbx, 128, 0, s, a, sx, n);
+    else pdl(flux_x_batched<CHQ_R, S, C, CHQ_P, 0>, nbx, 128, 0, s, a, sx, n);
   }
   return cudaGetLastError();
 }
