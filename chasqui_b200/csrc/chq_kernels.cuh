@@ -430,7 +430,8 @@ CHQ_D void fofc_flag_body(const FlagArgs &A, int bx, int by, int bz) {
     const double d = A.u[IDN * vs + l], m1 = A.u[IM1 * vs + l], m2 = A.u[IM2 * vs + l], m3 = A.u[IM3 * vs + l];
     const double en = A.u[IEN * vs + l];
     const double mm = 0.5 * (sqr(m1) + sqr(m2) + sqr(m3));
-    const double ke = in_range(d) ? quot(mm, d, rcp_n(d)) : divz(mm, d);
+    // (a momentum whose square or kinetic energy overflows makes p -inf, which is flagged)
+    const double ke = (in_range(d) && mm < 0x1p600) ? quot(mm, d, rcp_n(d)) : divz(mm, d);
     const double eint = en - ke - 0.5 * (bx * bx + by * by + bz * bz);
     double p = A.eos.gm1 * eint;
     if (A.eos.dual_energy && eint < A.eos.de_eta * fabs(en)) p = (A.u[IENT * vs + l] / d) * pow(d, A.eos.gamma);
@@ -939,7 +940,7 @@ template <class P, bool HST = false> CHQ_D void c2p_body(const C2pArgs<P> &A, in
     } else {
       p = fmax(p, e.pfloor);
       const double dg = pow(d, e.gamma);
-      sent = in_range(dg) ? quot(p, dg, rcp_n(dg)) : p / dg;
+      sent = (in_range(dg) && in_range(p)) ? quot(p, dg, rcp_n(dg)) : p / dg;
       A.u[IENT * vs + l] = d * sent;
     }
     A.w[IDN * vs + l] = P(d);
