@@ -405,7 +405,7 @@ CHQ_D bool face_solve(const FluxArgs<P> &A, const DirView<P> &V, int lf, const P
     } else {
       ok = ok && in_range(den) && in_range(cfmax);
       ratio = quot(num, den, rcp_n(den));
-      chi = quot(fmax_(flow_speed_q(L, b_n), flow_speed_q(R, b_n)), cfmax, rcp_n(cfmax));
+      chi = quot(fmax_(flow_speed_q(L, b_n, ok), flow_speed_q(R, b_n, ok)), cfmax, rcp_n(cfmax));
     }
     ratio = fmin_(P(1), ratio);
     chi = fmin_(P(1), chi);

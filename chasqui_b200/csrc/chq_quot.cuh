@@ -75,6 +75,8 @@ CHQ_DIV_HD bool in_range(float x) { return (unsigned)__float_as_int(x) - 0x2D800
 // the wider range of a lone quotient
 CHQ_DIV_HD bool quot_range(double x) { return in_range(x); }
 CHQ_DIV_HD bool quot_range(float x) { return (unsigned)__float_as_int(x) - 0x0F800000u < 0x60000000u; }
+CHQ_DIV_HD bool finite_q(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+CHQ_DIV_HD bool finite_q(float x) { return (__float_as_int(x) & 0x7f800000) != 0x7f800000; }
 CHQ_DIV_HD double fma_up(double a, double b, double c) { return __fma_ru(a, b, c); }
 CHQ_DIV_HD double fma_down(double a, double b, double c) { return __fma_rd(a, b, c); }
 // y with its last bit set when b's significand is all ones
@@ -109,6 +111,7 @@ inline bool in_range(double x) { return x >= 0x1p-300 && x < 0x1p+300; }
 inline bool in_range(float x) { return x >= 0x1p-36f && x < 0x1p+60f; }
 inline bool quot_range(double x) { return in_range(x); }
 inline bool quot_range(float x) { return x >= 0x1p-96f && x < 0x1p+96f; }
+template <class T> bool finite_q(T x) { return std::isfinite(x); }
 inline double fma_mode(int mode, double a, double b, double c) {
   const int old = std::fegetround();
   std::fesetround(mode);
@@ -186,6 +189,11 @@ template <class T> struct RootFloor;
 template <> struct RootFloor<double> { static constexpr double v = 0x1p-900; };
 template <> struct RootFloor<float> { static constexpr float v = 0x1p-120f; };
 
+// upper end of in_range
+template <class T> struct QuotMax;
+template <> struct QuotMax<double> { static constexpr double v = 0x1p+300; };
+template <> struct QuotMax<float> { static constexpr float v = 0x1p+60f; };
+
 // a / b for a >= 0, b > 0 (either may be out of range: then the plain division, out of line)
 #if defined(__CUDACC__)
 template <class T> __device__ __noinline__ T div_plain(T a, T b) { return a / b; }
@@ -194,7 +202,7 @@ template <class T> T div_plain(T a, T b) { return a / b; }
 #endif
 template <class T> CHQ_DIV_D T quot_pos(T a, T b) {
   const T r = quot(a, b, rcp_a(b));
-  return quot_range(b) ? r : div_plain(a, b);
+  return quot_range(b) && finite_q(a) ? r : div_plain(a, b);
 }
 
 // x / 6 and x / 12 with one product and the exact remainder (div6 in chq_divide.cuh has the

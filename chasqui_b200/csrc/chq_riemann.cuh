@@ -305,7 +305,7 @@ CHQ_HD void hlld(const MState<T> &L, const MState<T> &R, T bn, T gamma, T gm1, T
 // issue, so it evaluates only what the selected side needs: both sides' speeds and star
 // states, then the energies and the flux of one side. Every rounded operation has hlld's
 // operands, so the fluxes are the same; `ok` turns false when a divisor leaves the range the
-// quotients are exact in (vacuum, non-finite states, a degenerate negative star denominator),
+// quotients are exact in, or a numerator overflows (vacuum, non-finite states, a degenerate negative star denominator),
 // and the caller then evaluates hlld itself.
 
 // fast magnetosonic speed (fast_speed) from bsq = B^2
@@ -321,7 +321,7 @@ template <class T> CHQ_D T fast_speed_q(const MState<T> &s, T bn, T bsq, T gamma
 }
 
 // modified fast speed of LHLLD (flow_speed_u)
-template <class T> CHQ_D T flow_speed_q(const MState<T> &s, T bn) {
+template <class T> CHQ_D T flow_speed_q(const MState<T> &s, T bn, bool &ok) {
   const T vsq = s.u * s.u + s.v * s.v + s.w * s.w;
   const T yd = rcp_n(s.d);
   const T casq = quot(bn * bn + s.by * s.by + s.bz * s.bz, s.d, yd);
@@ -331,7 +331,8 @@ template <class T> CHQ_D T flow_speed_q(const MState<T> &s, T bn) {
   const T root = sqrt_q(disc);
   const T h = T(0.5) * (a + (disc > RootFloor<T>::v ? root : T(0)));
   const T r = sqrt_q(h);
-  return (h <= RootFloor<T>::v) ? T(0) : r;   // (a NaN stays one)
+  ok = ok && a < QuotMax<T>::v;   // (false for a NaN)
+  return (h <= RootFloor<T>::v) ? T(0) : r;
 }
 
 // single-star transverse velocity and field of one side (star_side); dm = rho (S - u), sms = S - S_M
@@ -474,7 +475,8 @@ CHQ_D bool hlld_q(const MState<T> &L, const MState<T> &R, T bn, T gm1, T rgm1, T
 #pragma unroll
     for (int n = 0; n < NFLX; ++n) f[n] = T(0.5) * (f[n] + f0[n]);
   }
-  return ok;
+  // a quotient of a numerator that overflowed is NaN, and so is then the energy flux
+  return ok && finite_q(f[FEN]);
 }
 
 }  // namespace chq

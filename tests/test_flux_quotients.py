@@ -3,7 +3,8 @@ states that reach each of its paths: ordinary shocks, gas at rest (both sides av
 field (single-star region), supersonic flow, and states whose divisors leave the range of the
 shared reciprocals, where the face is solved again with plain divisions, and a gas whose density,
 sound speed and field are a few units from 1, where quotients lie closest to rounding midpoints. One
-NaN cell must spread to the same faces. Ragged extents leave partial warps, tiles and march segments."""
+NaN cell must spread to the same faces, and so must velocities and fields that are infinite or whose
+squares overflow, in isolated cells. Ragged extents leave partial warps, tiles and march segments."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,7 @@ from chasqui_b200 import Mesh, make_config
 SHAPES = {"3d": (37, 9, 7), "2d": (66, 35, 1), "1d": (130, 1, 1)}
 SCHEMES = {"plm_hlld": (1, 1, 0), "ppm_hlld": (2, 1, 0), "wenoz_hlld": (3, 1, 0), "ppmx_lhlld": (4, 2, 0),
            "ppm_lhlld": (2, 2, 0), "ppm_hlld_char": (2, 1, 1), "wenoz_hlld_lowmach": (3, 1, 0)}
-KINDS = ("random", "rest", "rest_noise", "no_field", "supersonic", "stiff", "out_of_range", "nan", "near_one")
+KINDS = ("random", "rest", "rest_noise", "no_field", "supersonic", "stiff", "out_of_range", "nan", "near_one", "overflow", "infinite")
 
 
 def states(kind, shp, rng):
@@ -21,7 +22,7 @@ def states(kind, shp, rng):
     d, p = one.copy(), 0.1 * one
     v = [0.0 * one for _ in range(3)]
     b = [0.7 * one, 0.7 * one, 0.0 * one]
-    if kind in ("random", "nan", "stiff", "out_of_range"):
+    if kind in ("random", "nan", "stiff", "out_of_range", "overflow", "infinite"):
         d, p = 1.0 + rng.random(shp), 0.1 + rng.random(shp)
         v = [rng.normal(size=shp) for _ in range(3)]
         b = [rng.normal(size=shp) for _ in range(3)]
@@ -43,6 +44,14 @@ def states(kind, shp, rng):
             return a + rng.integers(-4, 3, shp) * 2.0 ** -53
         d, p = near(1.0), near(0.6)
         v, b = [rng.integers(-2, 3, shp) * 2.0 ** -50 for _ in range(3)], [near(1.0), near(0.0), near(0.0)]
+    b = [a.copy() for a in b]
+    if kind in ("overflow", "infinite"):   # one component in every seventh cell of each axis
+        k, j, i = np.indices(shp)
+        lone = (i % 7 == 3) & ((j % 7 == 3) | (shp[1] == 1)) & ((k % 7 == 3) | (shp[0] == 1))
+        big = rng.choice([1e80, 1e155, 1e160, -1e170] if kind == "overflow" else [np.inf, -np.inf], shp)
+        pick = rng.integers(0, 5, shp)
+        for q, a in enumerate(v + b[1:]):
+            a[:] = np.where(lone & (pick == q), big, a)
     w = np.stack([d, v[0], v[1], v[2], p, p / d ** (5.0 / 3.0)])
     if kind == "nan":
         w[1, shp[0] // 2, shp[1] // 2, shp[2] // 2] = np.nan
