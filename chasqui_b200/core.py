@@ -137,7 +137,7 @@ SIGNATURES = [
     ("chq_slab_end", C.c_int, [_P, _P]),
 ]
 
-TUNE_LENGTHS = (4, 8, 16, 32, 64)   # CHQ_TUNE_LENGTHS
+TUNE_LENGTHS = (1, 4, 16, 32, 64)   # CHQ_TUNE_LENGTHS
 TUNE_NLEN = len(TUNE_LENGTHS)
 TUNE_NXVAR = 2                       # CHQ_TUNE_NXVAR
 

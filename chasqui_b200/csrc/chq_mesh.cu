@@ -204,7 +204,7 @@ struct chq_mesh {
   int lo[3][3], hi[3][3], active[3];
   int act_lo[3][3], act_hi[3][3];
   int seglen;
-  bool march_set = false;   // set by the caller or a tuner (a batch then keeps it)
+  bool march_set = false;   // set by the caller or a tuner (a batch keeps it)
   int xvar = 0;   // x-sweep kernel variant (register cap), chq_autotune
   // y/z staging of the FP64 streaming-PPM march: 0 cp.async, 1 TMA (chq_autotune_yz); the
   // tensor maps over w and bcc are encoded at creation when the driver offers the encoder
@@ -1449,6 +1449,7 @@ struct chq_batch {
   std::vector<chq_mesh *> jobs;
   int mixed = 0, recon = 0, rsolver = 0, charac = 0, nstage = 0, fofc = 0, limiter = 0;
   int xvar = 0;   // x-sweep kernel variant of the batched flux launch (chq_batch_autotune)
+  int march = 0;  // march length of the members that have none of their own (batch_build)
   cudaStream_t stream = nullptr;
   char *dev = nullptr;
   struct Kind {
@@ -1523,17 +1524,16 @@ int batch_build(chq_batch *B) {
   const std::vector<chq_mesh *> &J = B->jobs;
   const int n = (int)J.size();
   // the members fill the device together, so the march length is chosen for all of them (a
-  // mesh's own default spreads it over the whole device), unless one was set or tuned
-  bool set = false;
-  for (const chq_mesh *m : J) set = set || m->march_set;
-  const int march = set ? 0 : default_march(J.data(), J.size());
+  // mesh's own default spreads it over the whole device); a member whose length was set or tuned keeps it
+  B->march = default_march(J.data(), J.size());
+  const auto march = [B](const chq_mesh *m) { return m->march_set ? 0 : B->march; };
   size_t o_flux_s, o_corner_s, o_update_s, o_flag_s, o_repair_s, o_limit_s, o_bc_s, o_c2p_s;
   o_flux_s = slots_of(h, J, [](chq_mesh *m) {
     const FluxArgs<P> a = flux_args<P>(m, 0, 7u);
     return linear((long)a.nxwarp * 32, 128);
   }, B->k_flux.nblocks);
   const size_t o_flux_yz_s = slots_of(h, J, [march](chq_mesh *m) {
-    const FluxArgs<P> a = flux_args<P>(m, 0, 7u, march);
+    const FluxArgs<P> a = flux_args<P>(m, 0, 7u, march(m));
     return linear((long)(a.nblk[1] + a.nblk[2]) * kYzThreads, kYzThreads);
   }, B->k_flux_yz.nblocks);
   o_corner_s = slots_of(h, J, [](chq_mesh *m) { return corner_grid(m); }, B->k_corner.nblocks);
@@ -1624,7 +1624,7 @@ int batch_build(chq_batch *B) {
       da[j] = diff_args<P>(m, bc1, bc2, bc3, &c->done, nd);
       ea[j] = res_emf_args<P>(m, bc1, bc2, bc3, &c->done, nullptr);
       ean[j] = res_emf_args<P>(m, bc1, bc2, bc3, &c->done, &c->nbad);
-      fa[j] = flux_args<P>(m, cur, 7u, march);
+      fa[j] = flux_args<P>(m, cur, 7u, march(m));
       fa[j].skip = &c->done;
       ua[j] = update_args<P>(m, out, g0, g1, 0.0, &c->beta_dt[st - 1], &c->done, nullptr);
       uan[j] = update_args<P>(m, out, g0, g1, 0.0, &c->beta_dt[st - 1], &c->done, &c->nbad);
@@ -3325,21 +3325,24 @@ int time_launches(cudaStream_t s, int reps, F launch, double *ms) {
 }
 
 // Two-knob search shared by meshes and batches: the y/z march length over CHQ_TUNE_LENGTHS
+// and the length the mesh or batch came with, own (0: none), so that tuning never ends on a slower one than that
 // (x-sweep variant 0), then the x-sweep variants at the best length (the knobs act on
 // different kernels). set(len, xvar) applies a candidate, run(&ms) times the flux launch.
 template <class Set, class Run>
-int tune_two_knobs(Set set, Run run, int nxvar, int *best_len, int *best_xvar, double ms_len[CHQ_TUNE_NLEN],
+int tune_two_knobs(Set set, Run run, int own, int nxvar, int *best_len, int *best_xvar, double ms_len[CHQ_TUNE_NLEN],
                    double ms_xvar[CHQ_TUNE_NXVAR]) {
-  const int cand[CHQ_TUNE_NLEN] = CHQ_TUNE_LENGTHS;
+  int cand[CHQ_TUNE_NLEN + 1] = CHQ_TUNE_LENGTHS;
+  int n = CHQ_TUNE_NLEN;
+  if (own > 0 && std::find(cand, cand + n, own) == cand + n) cand[n++] = own;
   double best = 1e300;
   *best_len = cand[0];
   *best_xvar = 0;
-  for (int q = 0; q < CHQ_TUNE_NLEN; ++q) {
+  for (int q = 0; q < n; ++q) {
     double t = 0.0;
     int rc = set(cand[q], 0);
     if (rc == CHQ_OK) rc = run(&t);
     if (rc != CHQ_OK) return rc;
-    if (ms_len) ms_len[q] = t;
+    if (ms_len && q < CHQ_TUNE_NLEN) ms_len[q] = t;
     if (t < best) {
       best = t;
       *best_len = cand[q];
@@ -3414,7 +3417,7 @@ int chq_autotune2(chq_mesh *m, int *seglen, int *xvar, double ms_len[CHQ_TUNE_NL
         return CHQ_OK;
       },
       [&](double *t) { return time_launches(s, 3, [&] { return do_fluxes(m, 0, 7u, nullptr, s); }, t); },
-      tune_xvariants(m->mixed), &bl, &bx, ms_len, ms_xvar);
+      keep_len, tune_xvariants(m->mixed), &bl, &bx, ms_len, ms_xvar);
   if (rc != CHQ_OK) {
     m->seglen = keep_len;
     m->xvar = keep_x;
@@ -3479,11 +3482,17 @@ int chq_batch_autotune(chq_batch *B, int *seglen, int *xvar, double ms_len[CHQ_T
     return (long)b;
   };
   const std::vector<long> key = {1, B->mixed, B->recon, B->rsolver, B->charac, lg(cells), lg((long)B->jobs.size())};
-  int bl = B->jobs[0]->seglen, bx = B->xvar;
+  // the length the batch came with (0: its members' lengths differ)
+  int own = -1;
+  for (const chq_mesh *m : B->jobs) {
+    const int len = m->march_set ? m->seglen : B->march;
+    own = (own < 0 || own == len) ? len : 0;
+  }
+  int bl = own > 0 ? own : B->march, bx = B->xvar;
   bool cached = false;
   if (cells >= kBatchTuneMaxCells) {
-    // the members' own settings already fill the device: no timing (it would cost more than
-    // it could gain over a short run); report them
+    // that length already fills the device: no timing (it would cost more than it could gain over a
+    // short run); report it
     if (ms_len)
       for (int q = 0; q < CHQ_TUNE_NLEN; ++q) ms_len[q] = -1.0;
     if (ms_xvar)
@@ -3533,7 +3542,7 @@ int chq_batch_autotune(chq_batch *B, int *seglen, int *xvar, double ms_len[CHQ_T
             return (e == cudaSuccess) ? CHQ_OK : cuda_fail(e, "batched flux launch");
           }, t);
         },
-        tune_xvariants(B->mixed), &bl, &bx, ms_len, ms_xvar);
+        own, tune_xvariants(B->mixed), &bl, &bx, ms_len, ms_xvar);
     if (rc != CHQ_OK) return rc;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune_cache[key] = {bl, bx};

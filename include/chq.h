@@ -227,7 +227,8 @@ CHQ_API int chq_profile(chq_mesh *m, int enable);
  *    compute the same bits, while in the mixed form the compiler may contract the FP32
  *    arithmetic of the two builds differently (chq_set_xvariant still selects it there).
  * chq_autotune2 times the flux launch of this mesh's scheme on its current state (call it
- * after chq_prime): every march length with variant 0, then every variant at the best length;
+ * after chq_prime): every march length, and the one the mesh came with where the list does not hold it
+ * (it is not among the returned times), with variant 0, then every variant at the best length;
  * it keeps the fastest pair on the mesh and returns it with the ms per launch of each
  * candidate (the arrays may be NULL). The choice is cached for the process per (precision,
  * reconstruction, Riemann solver, characteristic flag, nx1, nx2, nx3); a later mesh with the
@@ -236,12 +237,12 @@ CHQ_API int chq_profile(chq_mesh *m, int enable);
  * chq_batch_autotune does the same for a batch: it times the batched flux launch over all its
  * members (their march lengths and the batch's x variant change together; the batch's tables
  * are rebuilt for each candidate) and caches per (precision, scheme, log2 of the batch's
- * cells, log2 of its member count); a batch of 2^23 cells or more fills the device with its
- * members' own settings and is returned untimed (the arrays hold -1). A batch starts with the
- * march length that suits its members together, or with the members' own once one was set or
- * tuned, and with its first member's x variant. */
+ * cells, log2 of its member count); a batch of 2^23 cells or more fills the device with the
+ * length it came with and is returned untimed (the arrays hold -1). A batch starts with the
+ * march length that suits its members together, but for members whose length was set or
+ * tuned, which keep theirs, and with its first member's x variant. */
 #define CHQ_TUNE_NLEN 5
-#define CHQ_TUNE_LENGTHS {4, 8, 16, 32, 64}
+#define CHQ_TUNE_LENGTHS {1, 4, 16, 32, 64}
 #define CHQ_TUNE_NXVAR 2
 CHQ_API int chq_autotune(chq_mesh *m, int *seglen, double ms[CHQ_TUNE_NLEN]);
 CHQ_API int chq_autotune2(chq_mesh *m, int *seglen, int *xvar, double ms_len[CHQ_TUNE_NLEN],

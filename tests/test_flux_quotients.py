@@ -12,7 +12,7 @@ from chasqui_b200 import Mesh, make_config
 
 SHAPES = {"3d": (37, 9, 7), "2d": (66, 35, 1), "1d": (130, 1, 1)}
 SCHEMES = {"plm_hlld": (1, 1, 0), "ppm_hlld": (2, 1, 0), "wenoz_hlld": (3, 1, 0), "ppmx_lhlld": (4, 2, 0),
-           "ppm_lhlld": (2, 2, 0), "ppm_hlld_char": (2, 1, 1), "wenoz_hlld_lowmach": (3, 1, 0)}
+           "ppm_lhlld": (2, 2, 0), "plm_lhlld": (1, 2, 0), "ppm_hlld_char": (2, 1, 1), "wenoz_hlld_lowmach": (3, 1, 0)}
 KINDS = ("random", "rest", "rest_noise", "no_field", "supersonic", "stiff", "out_of_range", "nan", "near_one", "overflow", "infinite")
 
 

@@ -1,0 +1,67 @@
+"""Tuning never ends on a march length slower than the one it started from: the mesh's own length is
+among the candidates, a batch reports and keeps the length it uses, and one member with a length of
+its own does not change the others' results or lengths."""
+import numpy as np
+import pytest
+
+from chasqui_b200 import Batch, Mesh, make_config
+from chasqui_b200.core import TUNE_LENGTHS
+
+pytestmark = pytest.mark.gpu
+FIELDS = ("u0", "b1f0", "b2f0", "b3f0")
+
+
+def mesh(n, **kw):
+    m = Mesh(make_config(nx1=n[0], nx2=n[1], nx3=n[2], cfl=0.3, tlim=10.0, x1min=-.5, x1max=.5, x2min=-.5, x2max=.5,
+                         x3min=-.5, x3max=.5, **kw))
+    m.init_problem("blast", [10.0, 0.1, 0.2, 1.0, 30.0, 1e-2, 11])
+    m.prime(0.0)
+    return m
+
+
+def test_small_meshes_keep_short_marches():
+    """the default of a small mesh is one face a thread: it is a candidate, and four would be slower"""
+    m = mesh((60, 60, 1), recon=3)
+    assert m.seglen == 1 in TUNE_LENGTHS
+    r = m.autotune()
+    assert r["ms"][r["seglen"]] == min(r["ms"].values()) and r["ms"][1] <= r["ms"][4]
+    m.close()
+
+
+def test_the_own_length_is_a_candidate():
+    """a length outside the list is kept unless a listed one was measured faster"""
+    m = mesh((72, 70, 68), recon=3)
+    m.seglen = 5
+    r = m.autotune()
+    assert r["seglen"] == 5 or r["ms"][r["seglen"]] == min(r["ms"].values())
+    assert m.seglen == r["seglen"] and set(r["ms"]) == set(TUNE_LENGTHS)
+    m.close()
+
+
+def test_large_batches_report_the_length_they_use():
+    """2^23 cells or more are not timed; a small first member must not set the reported length"""
+    ms = [mesh((32, 32, 1))] + [mesh((128, 256, 136)) for _ in range(2)]
+    b = Batch(ms)
+    r = b.autotune()
+    assert ms[0].seglen == 1 and all(t < 0 for t in r["ms"].values())
+    assert r["seglen"] >= 8   # threads enough for the longest marches
+    b.close()
+    for m in ms:
+        m.close()
+
+
+def test_one_member_with_a_length_of_its_own():
+    shapes = [(20, 17, 11), (33, 31, 1), (18, 19, 20), (70, 1, 1)]
+    solo, members = [mesh(s) for s in shapes], [mesh(s) for s in shapes]
+    members[2].seglen = 7
+    b = Batch(members)
+    b.cycles(4)
+    b.status()
+    for a, m in zip(solo, members):
+        a.cycles(4)
+        for f in FIELDS:
+            assert np.array_equal(a.get(f), m.get(f)), f
+    assert [m.seglen for m in members] == [m.seglen for m in solo[:2]] + [7, solo[3].seglen]
+    b.close()
+    for m in solo + members:
+        m.close()
