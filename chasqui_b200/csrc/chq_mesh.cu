@@ -218,9 +218,9 @@ struct chq_mesh {
   // the FOFC repair reads the flags of the ghost plane below / above: only across an internal
   // slab boundary (at the periodic wrap the whole mesh's ghost cells are never flagged cells)
   int fofc_ext[2] = {0, 0};
-  // RKL2 work arrays (cfg.sts only): Y0..Y2, M0, Mj on cells; their face-field twins
-  double *sy[3] = {}, *sm0 = nullptr, *smj = nullptr;
-  double *sb[3][3] = {}, *smb0[3] = {}, *smbj[3] = {};
+  // RKL2 work arrays (cfg.sts only): Y1, Y2, M0, Mj on cells (Y0 is u0); their face-field twins
+  double *sy[2] = {}, *sm0 = nullptr, *smj = nullptr;
+  double *sb[2][3] = {}, *smb0[3] = {}, *smbj[3] = {};
   bool diff = false;
   long long sts_stages = 0;
   // set while the mesh is a member of a batch: the batch's end-of-cycles event, which every
@@ -307,8 +307,8 @@ const long kRepairBlocksBatched = 148;     // repair blocks per mesh of a batch
 // primitive type, the int flags, the control block and the history scratch
 size_t slab_size(size_t nel, size_t psize, bool sts) {
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-  // RKL2: 5 cell arrays of 6 components and 5 x 3 face fields, all double
-  const size_t sts_fields = sts ? 45 : 0;
+  // RKL2: Y1, Y2, M0 and Mj, each 6 cell components and 3 face fields, all double
+  const size_t sts_fields = sts ? 36 : 0;
   return nel * sizeof(double) * (18 + sts_fields) + nel * psize * 39 + up(nel * sizeof(int)) +
          up(kBadCap * sizeof(int)) + up(sizeof(StepCtl)) + up((size_t)(kHstBlocks * 10 + 16) * sizeof(double));
 }
@@ -1108,6 +1108,10 @@ int launch_spans(chq_mesh *m, const SpanArgs &a, cudaStream_t s) {
   return CHQ_OK;
 }
 
+// state buffers of the RKL2 stages: 0 is Y0 (u0 in place), 1 and 2 are Y1 and Y2, 3 is u1
+double *sts_cells(const chq_mesh *m, int b) { return b == 0 ? m->u[0] : b < 3 ? m->sy[b - 1] : m->u[1]; }
+double *sts_faces(const chq_mesh *m, int b, int d) { return b == 0 ? m->bf[0][d] : b < 3 ? m->sb[b - 1][d] : m->bf[1][d]; }
+
 // first component the diffusive terms change: the momenta with viscosity, else the energy only
 int sts_first_component(const chq_mesh *m) { return m->cfg.nu > 0.0 ? IM1 : IEN; }
 
@@ -1178,10 +1182,8 @@ int sts_advance(chq_mesh *m, double tau, double dt_par, cudaStream_t s, int &nst
   const double w1 = 4.0 / (double(ns) * ns + ns - 2.0);
   // Y0 is u0 itself: nothing writes it before the final copy but con2prim, whose entropy slot
   // is already what it writes
-  StsState Y0{m->u[0], {m->bf[0][0], m->bf[0][1], m->bf[0][2]}};
-  StsState Y1{m->sy[1], {m->sb[1][0], m->sb[1][1], m->sb[1][2]}};
-  StsState Y2{m->sy[2], {m->sb[2][0], m->sb[2][1], m->sb[2][2]}};
-  StsState spare{m->u[1], {m->bf[1][0], m->bf[1][1], m->bf[1][2]}};
+  auto state = [m](int b) { return StsState{sts_cells(m, b), {sts_faces(m, b, 0), sts_faces(m, b, 1), sts_faces(m, b, 2)}}; };
+  const StsState Y0 = state(0), Y1 = state(1), Y2 = state(2), spare = state(3);
   double *M0 = m->sm0, *Mj = m->smj;
   double *MB0[3] = {m->smb0[0], m->smb0[1], m->smb0[2]}, *MBj[3] = {m->smbj[0], m->smbj[1], m->smbj[2]};
   int rc;
@@ -1680,9 +1682,8 @@ int batch_build(chq_batch *B) {
     std::vector<StsDivArgs<P>> dv(n);
     std::vector<StsCombArgs> cb(n);
     std::vector<BcArgs> bb(n);
-    // Y0 is u0 in place, as in sts_advance
-    auto U = [](chq_mesh *m, int b) { return b == 0 ? m->u[0] : b < 3 ? m->sy[b] : m->u[1]; };
-    auto BF = [](chq_mesh *m, int b, int d) { return b == 0 ? m->bf[0][d] : b < 3 ? m->sb[b][d] : m->bf[1][d]; };
+    const auto U = sts_cells;
+    const auto BF = sts_faces;
     for (int b = 0; b < 4; ++b) {
       for (int j = 0; j < n; ++j) {
         chq_mesh *m = J[j];
@@ -1891,11 +1892,11 @@ int batch_sts(chq_batch *B, cudaStream_t s, long long &L) {
     const int b = wrote(ns);
     SpanArgs &f = fin[j];
     f.dst[0] = (unsigned long long *)m->u[0];
-    f.src[0] = (const unsigned long long *)(b < 3 ? m->sy[b] : m->u[1]);
+    f.src[0] = (const unsigned long long *)sts_cells(m, b);
     f.words[0] = NVAR * vs;
     for (int d = 0; d < 3; ++d) {
       f.dst[1 + d] = (unsigned long long *)m->bf[0][d];
-      f.src[1 + d] = (const unsigned long long *)(b < 3 ? m->sb[b][d] : m->bf[1][d]);
+      f.src[1 + d] = (const unsigned long long *)sts_faces(m, b, d);
       f.words[1 + d] = vs;
     }
     f.nspan = 4;
@@ -2291,10 +2292,10 @@ int mesh_create_impl(const chq_config *cfg, int nslab, int rank, chq_mesh **out)
   m->hst_out = m->hst_part + (size_t)m->hst_blocks * 10;
   p += align_up((size_t)(kHstBlocks * 10 + 16) * sizeof(double), 256);
   if (c.sts) {
-    for (int q = 0; q < 3; ++q) { m->sy[q] = (double *)p; p += dbytes * 6; }
+    for (int q = 0; q < 2; ++q) { m->sy[q] = (double *)p; p += dbytes * 6; }
     m->sm0 = (double *)p; p += dbytes * 6;
     m->smj = (double *)p; p += dbytes * 6;
-    for (int q = 0; q < 3; ++q)
+    for (int q = 0; q < 2; ++q)
       for (int d = 0; d < 3; ++d) { m->sb[q][d] = (double *)p; p += dbytes; }
     for (int d = 0; d < 3; ++d) { m->smb0[d] = (double *)p; p += dbytes; }
     for (int d = 0; d < 3; ++d) { m->smbj[d] = (double *)p; p += dbytes; }

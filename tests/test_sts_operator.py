@@ -42,3 +42,14 @@ def test_rkl2_cycles_equal_the_oracle(shape, coef):
     port.close()
     mesh.close()
     assert not bad, bad
+
+
+@pytest.mark.gpu
+def test_rkl2_scratch_is_four_states():
+    """Y1, Y2, M0 and Mj, nine double components a frame point each: Y0 is u0 itself"""
+    plain, sts = (Mesh(make_config(nx1=64, nx2=48, nx3=40, nu=0.1, sts=s)) for s in (0, 1))
+    pitch = -(-(64 + 2 * plain.ng + 1) // 32) * 32
+    points = -(-(40 + 2 * plain.ng + 1) * (48 + 2 * plain.ng + 1) * pitch // 64) * 64
+    assert sts.nbytes - plain.nbytes == 36 * 8 * points
+    for m in (plain, sts):
+        m.close()
