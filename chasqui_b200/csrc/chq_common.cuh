@@ -132,6 +132,8 @@ CHQ_D void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// set: the next launch starts a branch of a captured graph or depends on two, and is a plain one
+inline thread_local bool pdl_plain = false;
 template <class... KA, class... A>
 cudaError_t pdl(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchAttribute at{};
@@ -143,7 +145,8 @@ cudaError_t pdl(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaS
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &at;
-  cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= kPdlBlocks ? 1 : 0;
+  cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= kPdlBlocks && !pdl_plain ? 1 : 0;
+  pdl_plain = false;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 

@@ -280,8 +280,9 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_kern
 
 // K2 and K3 in one launch below 3-D, where a stage of a small mesh is mostly launches: each
 // point stores its edge EMFs and forms again the two neighbouring E3 its face fields need.
-// OT 64^2 90.9 -> 86.8 us a cycle, 256^2 131 -> 127 us; planes of more than kPlaneUpdatePoints
-// keep the two launches (1000^2 mixed: 853 us a cycle apart, 856 us in one). In 3-D the three
+// OT, us a cycle apart and in one: FP64 64^2 88.8 and 84.4, 256^2 125.8 and 123.4, 512^2 277 and 269,
+// 640^2 400 and 407, 768^2 552 and 558; mixed 64^2 82.5 and 77.5, 512^2 206 and 207, 640^2 295 and
+// 297, 768^2 381 and 391. Planes of more than kPlaneUpdatePoints (512^2) keep the two launches. In 3-D the three
 // EMFs of the neighbours cost more than the launch: a form that marched tiles up z and passed
 // them along took 2.4 ms where the two kernels take 1.5 at 256^3.
 constexpr long kPlaneUpdatePoints = 1L << 18;

@@ -6,14 +6,22 @@
 
 namespace chq {
 
+// While a cycle is captured into a graph: a second stream for the x sweep, which shares no data
+// with the y/z sweeps, and the events that fork it off and join it again
+struct FluxFork {
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+
+// fork: non-null while capturing (both sweeps then become parallel nodes where that pays)
 template <class P, int R>
-cudaError_t launch_flux(const FluxArgs<P> &a, int rsolver, int charac, cudaStream_t s);
+cudaError_t launch_flux(const FluxArgs<P> &a, int rsolver, int charac, const FluxFork *fork, cudaStream_t s);
 
 // x-sweep blocks and y/z-sweep blocks of many meshes, with one slot table each
 template <class P, int R>
 cudaError_t launch_flux_batched(const FluxArgs<P> *args, const BatchSlot *slots_x, const BatchSlot *slots_yz, int njobs,
                                 int rsolver, int charac, unsigned nblocks_x, unsigned nblocks_yz, int xvar,
-                                cudaStream_t s);
+                                const FluxFork *fork, cudaStream_t s);
 
 // registers per thread of the instantiated y/z kernel (for the launch report)
 template <class P, int R>

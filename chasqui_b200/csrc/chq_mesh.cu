@@ -205,6 +205,7 @@ struct chq_mesh {
   int act_lo[3][3], act_hi[3][3];
   int seglen;
   bool march_set = false;   // set by the caller or a tuner (a batch keeps it)
+  const chq::FluxFork *fork = nullptr;   // set while chq_cycles captures the cycle
   int xvar = 0;   // x-sweep kernel variant (register cap), chq_autotune
   // y/z staging of the FP64 streaming-PPM march: 0 cp.async, 1 TMA (chq_autotune_yz); the
   // tensor maps over w and bcc are encoded at creation when the driver offers the encoder
@@ -464,13 +465,13 @@ FluxArgs<P> flux_args(chq_mesh *m, int cur, unsigned dirmask, int march = 0) {
 }
 
 template <class P>
-cudaError_t launch_flux_any(const FluxArgs<P> &a, int recon, int rsolver, int charac, cudaStream_t s) {
+cudaError_t launch_flux_any(const FluxArgs<P> &a, int recon, int rsolver, int charac, const FluxFork *f, cudaStream_t s) {
   switch (recon) {
-    case R_DC: return launch_flux<P, R_DC>(a, rsolver, charac, s);
-    case R_PLM: return launch_flux<P, R_PLM>(a, rsolver, charac, s);
-    case R_PPM: return launch_flux<P, R_PPM>(a, rsolver, charac, s);
-    case R_PPMX: return launch_flux<P, R_PPMX>(a, rsolver, charac, s);
-    case R_WENOZ: return launch_flux<P, R_WENOZ>(a, rsolver, charac, s);
+    case R_DC: return launch_flux<P, R_DC>(a, rsolver, charac, f, s);
+    case R_PLM: return launch_flux<P, R_PLM>(a, rsolver, charac, f, s);
+    case R_PPM: return launch_flux<P, R_PPM>(a, rsolver, charac, f, s);
+    case R_PPMX: return launch_flux<P, R_PPMX>(a, rsolver, charac, f, s);
+    case R_WENOZ: return launch_flux<P, R_WENOZ>(a, rsolver, charac, f, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -481,11 +482,11 @@ int do_fluxes(chq_mesh *m, int cur, unsigned dirmask, const int *done, cudaStrea
   if (m->mixed) {
     FluxArgs<float> a = flux_args<float>(m, cur, dirmask);
     a.skip = done;
-    e = launch_flux_any(a, m->cfg.recon, m->cfg.rsolver, m->cfg.characteristic, s);
+    e = launch_flux_any(a, m->cfg.recon, m->cfg.rsolver, m->cfg.characteristic, m->fork, s);
   } else {
     FluxArgs<double> a = flux_args<double>(m, cur, dirmask);
     a.skip = done;
-    e = launch_flux_any(a, m->cfg.recon, m->cfg.rsolver, m->cfg.characteristic, s);
+    e = launch_flux_any(a, m->cfg.recon, m->cfg.rsolver, m->cfg.characteristic, m->fork, s);
   }
   if (e != cudaSuccess) return cuda_fail(e, "flux_kernel launch");
   return CHQ_OK;
@@ -1451,6 +1452,7 @@ struct chq_batch {
   std::vector<chq_mesh *> jobs;
   int mixed = 0, recon = 0, rsolver = 0, charac = 0, nstage = 0, fofc = 0, limiter = 0;
   int xvar = 0;   // x-sweep kernel variant of the batched flux launch (chq_batch_autotune)
+  const FluxFork *fork = nullptr;   // set while a cycle is captured
   int march = 0;  // march length of the members that have none of their own (batch_build)
   cudaStream_t stream = nullptr;
   char *dev = nullptr;
@@ -1829,11 +1831,11 @@ cudaError_t batch_flux(const chq_batch *B, const FluxArgs<P> *args, cudaStream_t
   const unsigned nbx = (unsigned)B->k_flux.nblocks, nbyz = (unsigned)B->k_flux_yz.nblocks;
   const BatchSlot *sx = B->k_flux.slots, *syz = B->k_flux_yz.slots;
   switch (B->recon) {
-    case R_DC: return launch_flux_batched<P, R_DC>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, s);
-    case R_PLM: return launch_flux_batched<P, R_PLM>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, s);
-    case R_PPM: return launch_flux_batched<P, R_PPM>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, s);
-    case R_PPMX: return launch_flux_batched<P, R_PPMX>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, s);
-    case R_WENOZ: return launch_flux_batched<P, R_WENOZ>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, s);
+    case R_DC: return launch_flux_batched<P, R_DC>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, B->fork, s);
+    case R_PLM: return launch_flux_batched<P, R_PLM>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, B->fork, s);
+    case R_PPM: return launch_flux_batched<P, R_PPM>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, B->fork, s);
+    case R_PPMX: return launch_flux_batched<P, R_PPMX>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, B->fork, s);
+    case R_WENOZ: return launch_flux_batched<P, R_WENOZ>(args, sx, syz, n, B->rsolver, B->charac, nbx, nbyz, B->xvar, B->fork, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -2795,6 +2797,24 @@ void clock_decode(const void *pinned, double *t, int *cycle) {
   *cycle = c->cycle;
 }
 
+// The second stream and events with which a capture makes the x sweep a branch of its own; the
+// graph outlives them. Without them the cycle is captured in series.
+struct CycleFork {
+  FluxFork f;
+  CycleFork() {
+    if (cudaStreamCreateWithFlags(&f.side, cudaStreamNonBlocking) != cudaSuccess) f.side = nullptr;
+    if (cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming) != cudaSuccess) f.fork = nullptr;
+    if (cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming) != cudaSuccess) f.join = nullptr;
+    if (!get()) cudaGetLastError();
+  }
+  ~CycleFork() {
+    if (f.fork) cudaEventDestroy(f.fork);
+    if (f.join) cudaEventDestroy(f.join);
+    if (f.side) cudaStreamDestroy(f.side);
+  }
+  const FluxFork *get() const { return f.side && f.fork && f.join ? &f : nullptr; }
+};
+
 void drop_cycle_graph(chq_mesh *m) {
   if (m->cyc_exec) cudaGraphExecDestroy(m->cyc_exec);
   if (m->cyc_graph) cudaGraphDestroy(m->cyc_graph);
@@ -2826,8 +2846,11 @@ int chq_cycles(chq_mesh *m, int n, void *stream) {
   if (done_plain == n) return CHQ_OK;
   if (!m->cyc_exec) {
     const long long l0 = m->nlaunch;
+    const CycleFork fork;
     CHQ_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    m->fork = fork.get();
     const int rc = plain_cycles(m, 1, s);
+    m->fork = nullptr;
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s, &g);
     if (rc) {
@@ -3230,8 +3253,11 @@ int chq_batch_cycles(chq_batch *B, int n, void *stream) {
   if (!B->exec) {
     // capture one cycle on the batch's own stream and keep the executable graph
     const long long l0 = B->nlaunch;
+    const CycleFork fork;
     CHQ_CUDA(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
+    B->fork = fork.get();
     const int rc = B->mixed ? batch_cycle<float>(B, B->stream) : batch_cycle<double>(B, B->stream);
+    B->fork = nullptr;
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(B->stream, &g);
     if (rc) {
