@@ -182,33 +182,37 @@ template <class P> struct PlaneEmf {
   CHQ_D double e3(long l) const { return (double)(A.g.two_d ? corner_e3(A, l) : ldg(A.e3x1 + l)); }
 };
 
+// the registers' weighted sum at l; ONE: of the first register alone, the other one's weight is zero
+template <bool ONE, class P> CHQ_D double mix(const UpdateArgs<P> &A, const double *a, const double *b, long l) {
+  return ONE ? A.g0 * a[l] : A.g0 * a[l] + A.g1 * b[l];
+}
+
 // new face fields; curl of the edge EMFs (src/physics.hpp:327-347)
-template <class P, class E> CHQ_D double new_b1(const UpdateArgs<P> &A, const E &em, long l, double g0, double g1, double bdt) {
+template <bool ONE, class P, class E> CHQ_D double new_b1(const UpdateArgs<P> &A, const E &em, long l, double bdt) {
   const Geom &g = A.g;
   double curl = 0.0;
   if (g.two_d) curl += (em.e3(l + g.sj) - em.e3(l)) * A.idx2;
   if (g.three_d) curl -= (em.e2(l + g.sk) - em.e2(l)) * A.idx3;
-  return g0 * A.b1a[l] + g1 * A.b1b[l] - bdt * curl;
+  return mix<ONE>(A, A.b1a, A.b1b, l) - bdt * curl;
 }
-template <class P, class E> CHQ_D double new_b2(const UpdateArgs<P> &A, const E &em, long l, double g0, double g1, double bdt) {
+template <bool ONE, class P, class E> CHQ_D double new_b2(const UpdateArgs<P> &A, const E &em, long l, double bdt) {
   const Geom &g = A.g;
   double curl = -(em.e3(l + 1) - em.e3(l)) * A.idx1;
   if (g.three_d) curl += (em.e1(l + g.sk) - em.e1(l)) * A.idx3;
-  return g0 * A.b2a[l] + g1 * A.b2b[l] - bdt * curl;
+  return mix<ONE>(A, A.b2a, A.b2b, l) - bdt * curl;
 }
-template <class P, class E> CHQ_D double new_b3(const UpdateArgs<P> &A, const E &em, long l, double g0, double g1, double bdt) {
+template <bool ONE, class P, class E> CHQ_D double new_b3(const UpdateArgs<P> &A, const E &em, long l, double bdt) {
   const Geom &g = A.g;
   double curl = (em.e2(l + 1) - em.e2(l)) * A.idx1;
   if (g.two_d) curl -= (em.e1(l + g.sj) - em.e1(l)) * A.idx2;
-  return g0 * A.b3a[l] + g1 * A.b3b[l] - bdt * curl;
+  return mix<ONE>(A, A.b3a, A.b3b, l) - bdt * curl;
 }
 
 // GRAV: compile the gravity epilogue (a separate instantiation keeps the plain update's
 // register count, and with it its occupancy, unchanged)
 // The update of one point (k, j, i) of the face/edge frame, is <= i <= ie+1 (and so on).
-template <class P, bool GRAV, class E> CHQ_D void update_point(const UpdateArgs<P> &A, const E &em, int k, int j, int i, double bdt) {
+template <class P, bool GRAV, bool ONE, class E> CHQ_D void update_point(const UpdateArgs<P> &A, const E &em, int k, int j, int i, double bdt) {
   const Geom &g = A.g;
-  const double g0 = A.g0, g1 = A.g1;
   const long l = g.idx(k, j, i);
   const long vs = g.vstride;
   const bool cell = (i <= g.ie && j <= g.je && k <= g.ke);
@@ -220,7 +224,7 @@ template <class P, bool GRAV, class E> CHQ_D void update_point(const UpdateArgs<
       double divf = ((double)ldg(A.f1 + ln + 1) - (double)ldg(A.f1 + ln)) * A.idx1;
       if (g.two_d) divf += ((double)ldg(A.f2 + ln + g.sj) - (double)ldg(A.f2 + ln)) * A.idx2;
       if (g.three_d) divf += ((double)ldg(A.f3 + ln + g.sk) - (double)ldg(A.f3 + ln)) * A.idx3;
-      un[n] = g0 * A.ua[ln] + g1 * A.ub[ln] - bdt * divf;
+      un[n] = mix<ONE>(A, A.ua, A.ub, ln) - bdt * divf;
     }
     if (GRAV && A.grav.on) {
       // ApplyGravity on the updated state with the stage primitives and beta*dt
@@ -244,9 +248,9 @@ template <class P, bool GRAV, class E> CHQ_D void update_point(const UpdateArgs<
     }
   }
   double nb1 = 0, nb2 = 0, nb3 = 0;
-  if (j <= g.je && k <= g.ke) nb1 = new_b1(A, em, l, g0, g1, bdt);
-  if (i <= g.ie && k <= g.ke && (g.two_d || j == g.js)) nb2 = new_b2(A, em, l, g0, g1, bdt);
-  if (i <= g.ie && j <= g.je && (g.three_d || k == g.ks)) nb3 = new_b3(A, em, l, g0, g1, bdt);
+  if (j <= g.je && k <= g.ke) nb1 = new_b1<ONE>(A, em, l, bdt);
+  if (i <= g.ie && k <= g.ke && (g.two_d || j == g.js)) nb2 = new_b2<ONE>(A, em, l, bdt);
+  if (i <= g.ie && j <= g.je && (g.three_d || k == g.ks)) nb3 = new_b3<ONE>(A, em, l, bdt);
   if (cell) {
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) A.uout[n * vs + l] = un[n];
@@ -262,7 +266,7 @@ template <class P, bool GRAV, class E> CHQ_D void update_point(const UpdateArgs<
   }
 }
 
-template <class P, bool GRAV = false> CHQ_D void update_body(const UpdateArgs<P> &A, int bx, int by, int bz) {
+template <class P, bool GRAV, bool ONE> CHQ_D void update_body(const UpdateArgs<P> &A, int bx, int by, int bz) {
   if (A.done && *A.done) return;
   if (A.need && *A.need <= A.need_min) return;
   const Geom &g = A.g;
@@ -270,12 +274,12 @@ template <class P, bool GRAV = false> CHQ_D void update_body(const UpdateArgs<P>
   const int j = g.js + by * blockDim.y + threadIdx.y;
   const int k = g.ks + bz;
   if (i > g.ie + 1 || j > g.je + 1 || k > g.ke + 1) return;
-  update_point<P, GRAV>(A, StoredEmf<P>{A}, k, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
+  update_point<P, GRAV, ONE>(A, StoredEmf<P>{A}, k, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
 }
 
-template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_kernel(const UpdateArgs<P> A) {
+template <class P, bool GRAV, bool ONE> __global__ void __launch_bounds__(256) update_kernel(const UpdateArgs<P> A) {
   pdl_begin();
-  update_body<P, GRAV>(A, blockIdx.x, blockIdx.y, blockIdx.z);
+  update_body<P, GRAV, ONE>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // K2 and K3 in one launch below 3-D, where a stage of a small mesh is mostly launches: each
@@ -286,7 +290,7 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_kern
 // EMFs of the neighbours cost more than the launch: a form that marched tiles up z and passed
 // them along took 2.4 ms where the two kernels take 1.5 at 256^3.
 constexpr long kPlaneUpdatePoints = 1L << 18;
-template <class P, bool GRAV>
+template <class P, bool GRAV, bool ONE>
 __global__ void __launch_bounds__(256) plane_update_kernel(const EmfArgs<P> E, const UpdateArgs<P> A) {
   pdl_begin();
   if (A.done && *A.done) return;
@@ -295,7 +299,7 @@ __global__ void __launch_bounds__(256) plane_update_kernel(const EmfArgs<P> E, c
   const int j = g.js + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ie + 1 || j > g.je + 1) return;
   corner_point<P>(E, g.ks, j, i);
-  update_point<P, GRAV>(A, PlaneEmf<P>{E}, g.ks, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
+  update_point<P, GRAV, ONE>(A, PlaneEmf<P>{E}, g.ks, j, i, A.beta_dt_dev ? *A.beta_dt_dev : A.beta_dt);
 }
 
 // FOFC re-run of the whole update: every point of the frame, blocks striding over its
@@ -310,7 +314,7 @@ template <class P, bool GRAV> CHQ_D void update_rerun_body(const UpdateArgs<P> &
   const long tiles = (long)nx * ny * nz;
   for (long t = b; t < tiles; t += nb) {
     const long r = t / nx;
-    update_body<P, GRAV>(A, (int)(t - r * nx), (int)(r % ny), (int)(r / ny));
+    update_body<P, GRAV, false>(A, (int)(t - r * nx), (int)(r % ny), (int)(r / ny));
   }
 }
 template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_rerun_kernel(const UpdateArgs<P> A) {
@@ -350,7 +354,7 @@ template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_reru
       const int j = jc + (p / 3) % rj - (rj >> 1);
       const int k = kc + p / (3 * rj) - (rk >> 1);
       if (i < g.is || i > g.ie + 1 || j < g.js || j > g.je + 1 || k < g.ks || k > g.ke + 1) continue;
-      update_point<P, GRAV>(A, StoredEmf<P>{A}, k, j, i, bdt);
+      update_point<P, GRAV, false>(A, StoredEmf<P>{A}, k, j, i, bdt);
     }
   }
 }
@@ -1113,14 +1117,14 @@ template <class P> __global__ void __launch_bounds__(256) corner_rerun_batched(c
   const EmfArgs<P> &A = stage_args(args, j, sa);
   corner_rerun_body<P>(A, (int)(blockIdx.x - slots[j].off), slots[j].gx);
 }
-template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_batched(const UpdateArgs<P> *args, const BatchSlot *slots, int n) {
+template <class P, bool GRAV, bool ONE> __global__ void __launch_bounds__(256) update_batched(const UpdateArgs<P> *args, const BatchSlot *slots, int n) {
   pdl_begin();
   int bx, by, bz;
   const int j = batch_job(slots, n, blockIdx.x);
   batch_block(slots[j], blockIdx.x, bx, by, bz);
   __shared__ __align__(16) unsigned char sa[sizeof(UpdateArgs<P>)];
   const UpdateArgs<P> &A = stage_args(args, j, sa);
-  update_body<P, GRAV>(A, bx, by, bz);
+  update_body<P, GRAV, ONE>(A, bx, by, bz);
 }
 template <class P, bool GRAV> __global__ void __launch_bounds__(256) update_rerun_batched(const UpdateArgs<P> *args, const BatchSlot *slots, int n) {
   pdl_begin();

@@ -549,6 +549,9 @@ int do_corner_rerun(chq_mesh *m, const int *done, const int *need, cudaStream_t 
 }
 
 // ---- update --------------------------------------------------------------------------
+// weights of which one is zero (the update's first pass then reads one register)
+bool one_register(double g0, double g1) { return (g0 == 0.0) != (g1 == 0.0); }
+
 template <class P>
 UpdateArgs<P> update_args(chq_mesh *m, int out, double g0, double g1, double bdt, const double *bdt_dev,
                           const int *done, const int *need) {
@@ -558,16 +561,16 @@ UpdateArgs<P> update_args(chq_mesh *m, int out, double g0, double g1, double bdt
   a.eos = m->eos;
   a.f1 = as<P>(m->flx[0]); a.f2 = as<P>(m->flx[1]); a.f3 = as<P>(m->flx[2]);
   a.e1 = as<P>(m->e[0]); a.e2 = as<P>(m->e[1]); a.e3 = as<P>(m->e[2]);
-  // A register with a zero weight adds a zero whatever it holds: the first pass takes that zero
-  // from the other register, whose lines it reads anyway, and so reads 72 of 384 bytes a cell
-  // less in the first stage of RK2, RK3 and SSPRK(4,3). A re-run keeps both (its b-register may
-  // hold a first pass that was not finite, which has to stay so).
-  const int ia = (!need && g0 == 0.0) ? 1 : 0, ib = (!need && g1 == 0.0) ? 0 : 1;
-  a.ua = m->u[ia]; a.ub = m->u[ib]; a.uout = m->u[out];
+  // A register with a zero weight would add a zero: the first pass does not read it (the kernels'
+  // ONE form), 72 of 384 bytes a cell less in the first stage of RK2, RK3 and SSPRK(4,3). A re-run
+  // keeps both (its b-register may hold a first pass that was not finite, which has to stay so).
+  const bool one = !need && one_register(g0, g1);
+  const int ia = (one && g0 == 0.0) ? 1 : 0;
+  a.ua = m->u[ia]; a.ub = m->u[1]; a.uout = m->u[out];
   a.b1a = m->bf[ia][0]; a.b2a = m->bf[ia][1]; a.b3a = m->bf[ia][2];
-  a.b1b = m->bf[ib][0]; a.b2b = m->bf[ib][1]; a.b3b = m->bf[ib][2];
+  a.b1b = m->bf[1][0]; a.b2b = m->bf[1][1]; a.b3b = m->bf[1][2];
   a.b1o = m->bf[out][0]; a.b2o = m->bf[out][1]; a.b3o = m->bf[out][2];
-  a.g0 = g0; a.g1 = g1; a.beta_dt = bdt; a.beta_dt_dev = bdt_dev;
+  a.g0 = one ? g0 + g1 : g0; a.g1 = g1; a.beta_dt = bdt; a.beta_dt_dev = bdt_dev;
   a.idx1 = 1.0 / g.dx1; a.idx2 = 1.0 / g.dx2; a.idx3 = 1.0 / g.dx3;
   a.done = done;
   a.need = need;
@@ -596,8 +599,9 @@ int do_update(chq_mesh *m, int out, double g0, double g1, double bdt, const doub
   const UpdateArgs<P> a = update_args<P>(m, out, g0, g1, bdt, bdt_dev, done, nullptr);
   const Launch3 L = update_grid(m);
   m->nlaunch += 1;
-  if (a.grav.on) pdl(update_kernel<P, true>, L.grid, L.block, 0, s, a);
-  else pdl(update_kernel<P, false>, L.grid, L.block, 0, s, a);
+  const bool one = one_register(g0, g1);
+  if (a.grav.on) pdl(one ? update_kernel<P, true, true> : update_kernel<P, true, false>, L.grid, L.block, 0, s, a);
+  else pdl(one ? update_kernel<P, false, true> : update_kernel<P, false, false>, L.grid, L.block, 0, s, a);
   CHQ_CUDA(cudaGetLastError());
   return CHQ_OK;
 }
@@ -610,8 +614,11 @@ int do_plane_update(chq_mesh *m, int out, double g0, double g1, double bdt, cons
   const UpdateArgs<P> a = update_args<P>(m, out, g0, g1, bdt, bdt_dev, done, nullptr);
   const Launch3 L = update_grid(m);
   m->nlaunch += 1;
-  if (a.grav.on) CHQ_CUDA(pdl(plane_update_kernel<P, true>, L.grid, L.block, 0, s, e, a));
-  else CHQ_CUDA(pdl(plane_update_kernel<P, false>, L.grid, L.block, 0, s, e, a));
+  const bool one = one_register(g0, g1);
+  if (a.grav.on)
+    CHQ_CUDA(pdl(one ? plane_update_kernel<P, true, true> : plane_update_kernel<P, true, false>, L.grid, L.block, 0, s, e, a));
+  else
+    CHQ_CUDA(pdl(one ? plane_update_kernel<P, false, true> : plane_update_kernel<P, false, false>, L.grid, L.block, 0, s, e, a));
   return CHQ_OK;
 }
 
@@ -1984,10 +1991,14 @@ int batch_cycle(chq_batch *B, cudaStream_t s) {
       ++L;
     }
     auto update = [&](const void *args) -> cudaError_t {
-      if (B->grav)
-        pdl(update_batched<P, true>, (unsigned)B->k_update.nblocks, b2, 0, s, (const UpdateArgs<P> *)args, B->k_update.slots, n);
-      else
-        pdl(update_batched<P, false>, (unsigned)B->k_update.nblocks, b2, 0, s, (const UpdateArgs<P> *)args, B->k_update.slots, n);
+      double g0, g1, beta;
+      int cur, out;
+      stage_table(B->nstage, st + 1, g0, g1, beta, cur, out);
+      const bool one = one_register(g0, g1);
+      const unsigned nb = (unsigned)B->k_update.nblocks;
+      const UpdateArgs<P> *a = (const UpdateArgs<P> *)args;
+      if (B->grav) pdl(one ? update_batched<P, true, true> : update_batched<P, true, false>, nb, b2, 0, s, a, B->k_update.slots, n);
+      else pdl(one ? update_batched<P, false, true> : update_batched<P, false, false>, nb, b2, 0, s, a, B->k_update.slots, n);
       ++L;
       return cudaGetLastError();
     };

@@ -1,6 +1,6 @@
 """The update reads a register of zero weight through the other one: every pair of weights the
-integrators use and each output register, registers that differ, against the plain-C oracle
-(FP64, state and face fields bit for bit)."""
+integrators use and each output register, registers that differ and hold infinities, against the
+plain-C oracle (FP64, state and face fields bit for bit)."""
 import numpy as np
 import pytest
 
@@ -27,16 +27,21 @@ def test_update_weights_equal_the_oracle(shape):
     portsim.lib().port_corner_emf(port._h)
     rng = np.random.default_rng(3)
     regs = {f + "%d" % r: rng.normal(size=mesh.shape(f + "%d" % r)) for f in ("u", "b1f", "b2f", "b3f") for r in (0, 1)}
+    for f in [f for f in regs if f[0] == "u"]:   # values that a product with zero would not leave alone
+        regs[f][:, :, :, 6] = np.inf
+        regs[f][:, :, :, 9] = -np.inf
     bad = {}
     for g0, g1, out in WEIGHTS:
         for f, a in regs.items():
+            if g0 * g1 == 0.0 and f.endswith("1" if g1 == 0.0 else "0"):
+                a = np.where(np.isfinite(a), a, 1.0)   # (the oracle multiplies the register of zero weight too)
             mesh.set(f, a)
             port.set(f, a)
         mesh.update(out, g0, g1, 1e-3)
         portsim.lib().port_update(port._h, out, g0, g1, 1e-3)
         for f in ("u%d", "b1f%d", "b2f%d", "b3f%d"):
             got, want = mesh.get(f % out).ravel(), port.get(f % out)
-            if not np.array_equal(got, want):
+            if not np.array_equal(got, want, equal_nan=True):
                 bad[(g0, g1, out, f)] = (int((got != want).sum()), float(np.abs(got - want).max()))
     port.close()
     mesh.close()
