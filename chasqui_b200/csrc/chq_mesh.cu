@@ -3369,6 +3369,35 @@ int time_launches(cudaStream_t s, int reps, F launch, double *ms) {
   return CHQ_OK;
 }
 
+// Device time of `launch` as a captured cycle runs it, the x sweep a branch of its own: replays of
+// a graph of it (20 of a short one). *slot is the mesh's or batch's fork pointer.
+template <class F>
+int time_replays(cudaStream_t s, const FluxFork **slot, F launch, double *ms) {
+  const CycleFork fork;
+  int rc = launch();   // loads the kernels before the capture
+  if (rc != CHQ_OK) return rc;
+  CHQ_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  *slot = fork.get();
+  rc = launch();
+  *slot = nullptr;
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamEndCapture(s, &g);
+  cudaGraphExec_t exec = nullptr;
+  if (rc == CHQ_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
+  auto replay = [&] {
+    const cudaError_t r = cudaGraphLaunch(exec, s);
+    return r == cudaSuccess ? CHQ_OK : cuda_fail(r, "autotune timing");
+  };
+  if (exec) {
+    rc = time_launches(s, 3, replay, ms);
+    if (rc == CHQ_OK && *ms < 0.1) rc = time_launches(s, 20, replay, ms);
+    cudaGraphExecDestroy(exec);
+  }
+  if (g) cudaGraphDestroy(g);
+  if (rc == CHQ_OK && e != cudaSuccess) return cuda_fail(e, "autotune timing");
+  return rc;
+}
+
 // Two-knob search shared by meshes and batches: the y/z march length over CHQ_TUNE_LENGTHS
 // and the length the mesh or batch came with, own (0: none), so that tuning never ends on a slower one than that
 // (x-sweep variant 0), then the x-sweep variants at the best length (the knobs act on
@@ -3461,7 +3490,11 @@ int chq_autotune2(chq_mesh *m, int *seglen, int *xvar, double ms_len[CHQ_TUNE_NL
         m->xvar = v;
         return CHQ_OK;
       },
-      [&](double *t) { return time_launches(s, 3, [&] { return do_fluxes(m, 0, 7u, nullptr, s); }, t); },
+      [&](double *t) {
+        auto launch = [&] { return do_fluxes(m, 0, 7u, nullptr, s); };
+        if (m->cfg.sts && m->diff) return time_launches(s, 3, launch, t);   // cycles without a graph
+        return time_replays(s, &m->fork, launch, t);
+      },
       keep_len, tune_xvariants(m->mixed), &bl, &bx, ms_len, ms_xvar);
   if (rc != CHQ_OK) {
     m->seglen = keep_len;
@@ -3581,11 +3614,13 @@ int chq_batch_autotune(chq_batch *B, int *seglen, int *xvar, double ms_len[CHQ_T
     const int rc = tune_two_knobs(
         set,
         [&](double *t) {
-          return time_launches(B->stream, 3, [&]() -> int {
+          auto launch = [&]() -> int {
             const cudaError_t e = B->mixed ? batch_flux<float>(B, (const FluxArgs<float> *)B->a_flux[0], B->stream)
                                            : batch_flux<double>(B, (const FluxArgs<double> *)B->a_flux[0], B->stream);
             return (e == cudaSuccess) ? CHQ_OK : cuda_fail(e, "batched flux launch");
-          }, t);
+          };
+          if (B->sts || !B->use_graph) return time_launches(B->stream, 3, launch, t);
+          return time_replays(B->stream, &B->fork, launch, t);
         },
         own, tune_xvariants(B->mixed), &bl, &bx, ms_len, ms_xvar);
     if (rc != CHQ_OK) return rc;

@@ -28,6 +28,30 @@ def test_small_meshes_keep_short_marches():
     m.close()
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+def test_tuned_cycles_are_not_slower(precision):
+    """what is timed is what a captured cycle runs (the sweeps side by side): whole cycles with the tuned
+    length within a twentieth of the default's, the best of several"""
+    import time
+    best = {}
+    for tuned in (False, True):
+        m = mesh((256, 256, 1), precision=precision)
+        if tuned:
+            m.autotune()
+        m.cycles(4)
+        m.clock()
+        best[tuned] = min(timed(m, time.perf_counter) for _ in range(8))
+        m.close()
+    assert best[True] <= 1.05 * best[False], best
+
+
+def timed(m, now):
+    t = now()
+    m.cycles(50)
+    m.clock()
+    return now() - t
+
+
 def test_the_own_length_is_a_candidate():
     """a length outside the list is kept unless a listed one was measured faster"""
     m = mesh((72, 70, 68), recon=3)
