@@ -31,7 +31,8 @@
 // tests/test_quot.py compares all of them with the IEEE operations, on the device and, with
 // coarser seeds, on the host.
 // Valid for finite numerators and for divisors and radicands that in_range accepts (FP64
-// 2^-300 .. 2^300, FP32 2^-36 .. 2^60, positive); outside it the caller takes
+// 2^-300 .. 2^300, FP32 2^-60 .. 2^60, positive: in FP32 the square of a divisor and that of its
+// reciprocal are then normal numbers); outside it the caller takes
 // the plain operations. Compiles for the host as well, with the seeds emulated: 20 bits in FP64,
 // and in FP32 a reciprocal one unit above and a root of 22 bits.
 #pragma once
@@ -71,7 +72,7 @@ CHQ_DIV_HD float rsqrt_seed(float b) {
   return y;
 }
 CHQ_DIV_HD bool in_range(double x) { return (unsigned)__double2hiint(x) - 0x2D300000u < 0x25800000u; }
-CHQ_DIV_HD bool in_range(float x) { return (unsigned)__float_as_int(x) - 0x2D800000u < 0x30000000u; }
+CHQ_DIV_HD bool in_range(float x) { return (unsigned)__float_as_int(x) - 0x21800000u < 0x3C000000u; }
 // the wider range of a lone quotient
 CHQ_DIV_HD bool quot_range(double x) { return in_range(x); }
 CHQ_DIV_HD bool quot_range(float x) { return (unsigned)__float_as_int(x) - 0x0F800000u < 0x60000000u; }
@@ -108,7 +109,7 @@ inline float rcp_seed(float b) {   // one unit at most, from above
 }
 inline float rsqrt_seed(float b) { return (float)chop(1.0 / ::sqrt((double)b), 22); }
 inline bool in_range(double x) { return x >= 0x1p-300 && x < 0x1p+300; }
-inline bool in_range(float x) { return x >= 0x1p-36f && x < 0x1p+60f; }
+inline bool in_range(float x) { return x >= 0x1p-60f && x < 0x1p+60f; }
 inline bool quot_range(double x) { return in_range(x); }
 inline bool quot_range(float x) { return x >= 0x1p-96f && x < 0x1p+96f; }
 template <class T> bool finite_q(T x) { return std::isfinite(x); }

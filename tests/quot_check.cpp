@@ -56,7 +56,7 @@ template <class T> static long run(long n, int elo, int ehi, const char *name) {
 int main(int argc, char **argv) {
   const long n = argc > 1 ? std::atol(argv[1]) : 2000000;
   if (run<double>(n, -300, 300, "double") || run<double>(n, -3, 3, "double near one")) return 1;
-  if (run<float>(n, -30, 30, "float") || run<float>(n, -3, 3, "float near one")) return 1;
+  if (run<float>(n, -60, 60, "float") || run<float>(n, -3, 3, "float near one")) return 1;
   if (off * 10000 > 2 * n) return std::printf("float: %ld of %ld results one unit off\n", off, 2 * n), 1;
   std::printf("ok %ld\n", 4 * n);
   return 0;
