@@ -180,8 +180,8 @@ def run_form(n, precision, steps, warmup, dist, device, sample_clocks=False, pro
     mesh = Mesh(blast_config(n, precision))
     mesh.init_problem("blast", BLAST_PARAMS)
     mesh.prime(0.0)
-    # flux-kernel march length picked by the library's autotuner on this state (the default
-    # is 16; the per-length launch times are reported beside the choice). `pin` =
+    # flux-kernel march length picked by the library's autotuner on this state (the mesh's own
+    # default is a candidate; the listed lengths' launch times are reported beside the choice). `pin` =
     # (march length, x variant, y/z staging) skips the tuner and sets those, so that a run
     # under a profiler, whose serialised replays distort the tuner's timings, launches the
     # kernels a plain run picked.

@@ -329,11 +329,11 @@ template <int RE, class P> struct WindowStencil {
 // ---------------------------------------------------------------------------------------
 // Face work: Riemann solve of the face `lf` (between cells lf - stride and lf).
 //
-// What bounds it: FP64 issue (61 % of the FP64 pipe's cycles in the y/z launch, 68 % in the x
-// launch at 128^3; 730 FP64 operations a face and thread). With compiled divisions and branching
+// What bounds it: FP64 issue (61 % of the FP64 pipe's cycles in the y/z launch, 70 % in the x
+// launch at 128^3; 746 FP64 operations a face and thread). With compiled divisions and branching
 // limiters a face took 2200 warp instructions at 24 of 32 active lanes and waited on instruction
 // fetch; with chq_quot.cuh and selects it takes 1380 at 31.6, and the FP64 PPM + HLLD flux launch
-// went from 0.880 to 0.444 ms at 128^3 (blast), 5.21 to 3.20 ms at 256^3 (mixed: 2.89 to 1.85 ms),
+// went from 0.880 to 0.45 ms at 128^3 (blast), 5.21 to 3.24 ms at 256^3 (mixed: 2.89 to 1.85 ms),
 // WENO-Z from 1.92 to 0.78 ms at 128^3, OT 256^2 from 43 to 16 us (rows laid end to end and
 // balanced marches included).
 

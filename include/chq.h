@@ -209,7 +209,8 @@ CHQ_API int chq_event_elapsed_between(chq_mesh *ma, int a, chq_mesh *mb, int b, 
 /* Per-kernel CUDA-event timing inside the stage sequence (off by default). Kinds:
  * 0 fluxes (K1), 1 corner EMF (K2), 2 update (K3), 3 FOFC flag, 4 FOFC repair + re-run,
  * 5 boundaries (K4), 6 con2prim + dt (K5), 7 positivity limiter, 8 step control,
- * 9 explicit diffusion (diffusive fluxes, resistive EMF, density minimum), 10 RKL2 super-step. */
+ * 9 explicit diffusion (diffusive fluxes, resistive EMF, density minimum), 10 RKL2 super-step.
+ * Below 3-D, planes of at most 2^18 points form their corner EMFs inside the update (kind 2). */
 #define CHQ_NPROF 11
 /* Number of CUDA kernels this mesh has launched so far (including early-exit launches). */
 CHQ_API long long chq_kernel_launches(const chq_mesh *m);
