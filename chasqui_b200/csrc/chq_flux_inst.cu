@@ -25,8 +25,8 @@ static cudaError_t allow_smem(K kern, size_t smem, bool *ready) {
   return e;
 }
 
-// In a captured cycle the x sweep is a parallel node of the y/z sweeps up to this many x blocks: its
-// blocks fill what the y/z launch's last waves leave idle. us a cycle in series and in parallel: OT 64^2
+// In a captured cycle the x sweep is a parallel node of the y/z sweeps up to this many x blocks (in
+// cycles without a graph it runs on the mesh's second stream): its blocks fill what the y/z launch's last waves leave idle. us a cycle in series and in parallel: OT 64^2
 // 94 and 82, 256^2 154 and 122, 512^2 279 and 269, 128^3 2313 and 2288 (mixed 96, 87 at 128^2, 221, 207
 // at 512^2, 1674, 1584 at 128^3); 256^3, whose two launches are many waves each, 16 635 and 16 660
 // (11 255 and 11 301).

@@ -6,14 +6,14 @@
 
 namespace chq {
 
-// While a cycle is captured into a graph: a second stream for the x sweep, which shares no data
-// with the y/z sweeps, and the events that fork it off and join it again
+// A second stream for the x sweep, which shares no data with the y/z sweeps, and the events that
+// fork it off and join it again (while a cycle is captured, or in cycles without a graph)
 struct FluxFork {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
 
-// fork: non-null while capturing (both sweeps then become parallel nodes where that pays)
+// fork: when given, both sweeps run side by side where that pays
 template <class P, int R>
 cudaError_t launch_flux(const FluxArgs<P> &a, int rsolver, int charac, const FluxFork *fork, cudaStream_t s);
 

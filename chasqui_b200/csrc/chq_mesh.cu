@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <mutex>
 #include "chq.h"
 #include "chq_common.cuh"
@@ -171,6 +172,27 @@ __global__ void hst_final_kernel(const double *part, int nblk, double *out) {
 }
 }  // namespace chq
 
+namespace chq {
+// The second stream and events with which the x sweep runs beside the y/z sweeps: as a branch of a
+// captured cycle (the graph outlives them), or in a mesh's cycles without a graph. Where they cannot
+// be made the sweeps run in series.
+struct CycleFork {
+  FluxFork f;
+  CycleFork() {
+    if (cudaStreamCreateWithFlags(&f.side, cudaStreamNonBlocking) != cudaSuccess) f.side = nullptr;
+    if (cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming) != cudaSuccess) f.fork = nullptr;
+    if (cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming) != cudaSuccess) f.join = nullptr;
+    if (!get()) cudaGetLastError();
+  }
+  ~CycleFork() {
+    if (f.fork) cudaEventDestroy(f.fork);
+    if (f.join) cudaEventDestroy(f.join);
+    if (f.side) cudaStreamDestroy(f.side);
+  }
+  const FluxFork *get() const { return f.side && f.fork && f.join ? &f : nullptr; }
+};
+}  // namespace chq
+
 // ---------------------------------------------------------------------------------------
 struct chq_mesh {
   chq_config cfg;
@@ -205,7 +227,8 @@ struct chq_mesh {
   int act_lo[3][3], act_hi[3][3];
   int seglen;
   bool march_set = false;   // set by the caller or a tuner (a batch keeps it)
-  const chq::FluxFork *fork = nullptr;   // set while chq_cycles captures the cycle
+  const chq::FluxFork *fork = nullptr;   // set while chq_cycles captures or launches cycles
+  std::unique_ptr<chq::CycleFork> own_fork;   // of cycles that are never captured (RKL2, a caller's stream)
   int xvar = 0;   // x-sweep kernel variant (register cap), chq_autotune
   // y/z staging of the FP64 streaming-PPM march: 0 cp.async, 1 TMA (chq_autotune_yz); the
   // tensor maps over w and bcc are encoded at creation when the driver offers the encoder
@@ -2808,24 +2831,6 @@ void clock_decode(const void *pinned, double *t, int *cycle) {
   *cycle = c->cycle;
 }
 
-// The second stream and events with which a capture makes the x sweep a branch of its own; the
-// graph outlives them. Without them the cycle is captured in series.
-struct CycleFork {
-  FluxFork f;
-  CycleFork() {
-    if (cudaStreamCreateWithFlags(&f.side, cudaStreamNonBlocking) != cudaSuccess) f.side = nullptr;
-    if (cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming) != cudaSuccess) f.fork = nullptr;
-    if (cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming) != cudaSuccess) f.join = nullptr;
-    if (!get()) cudaGetLastError();
-  }
-  ~CycleFork() {
-    if (f.fork) cudaEventDestroy(f.fork);
-    if (f.join) cudaEventDestroy(f.join);
-    if (f.side) cudaStreamDestroy(f.side);
-  }
-  const FluxFork *get() const { return f.side && f.fork && f.join ? &f : nullptr; }
-};
-
 void drop_cycle_graph(chq_mesh *m) {
   if (m->cyc_exec) cudaGraphExecDestroy(m->cyc_exec);
   if (m->cyc_graph) cudaGraphDestroy(m->cyc_graph);
@@ -2846,7 +2851,18 @@ int chq_cycles(chq_mesh *m, int n, void *stream) {
   if (m->slab_count > 1) return fail(CHQ_ERR_ARG, "a z slab steps through chq_slab_begin / chq_slab_stage / chq_slab_end");
   cudaStream_t s = S(m, stream);
   const bool graphable = !(m->cfg.sts && m->diff) && !m->prof && (stream == nullptr || s == m->stream);
-  if (!graphable || n == 0) return plain_cycles(m, n, s);
+  if (!graphable || n == 0) {
+    // (not into a caller's capture, and not under per-kernel timing)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CHQ_CUDA(cudaStreamIsCapturing(s, &capture));
+    if (n > 0 && !m->prof && capture == cudaStreamCaptureStatusNone) {
+      if (!m->own_fork) m->own_fork = std::make_unique<CycleFork>();
+      m->fork = m->own_fork->get();
+    }
+    const int rc = plain_cycles(m, n, s);
+    m->fork = nullptr;
+    return rc;
+  }
   int done_plain = 0;
   if (!m->cyc_warm) {
     const int rc = plain_cycles(m, 1, s);

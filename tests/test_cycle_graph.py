@@ -35,6 +35,28 @@ def test_replayed_cycles_equal_launches(shape, precision):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
+def test_cycles_on_a_callers_stream_equal_replayed_ones(precision):
+    """no graph there: the sweeps run side by side on the mesh's second stream, joined by events"""
+    import ctypes
+    import torch
+    from chasqui_b200.core import load_library
+    a, b = (mesh((66, 35, 1), precision, 2) for _ in range(2))
+    c, d = (mesh((37, 40, 33), precision, 3) for _ in range(2))
+    s = torch.cuda.Stream()
+    for m in (b, d):
+        for _ in range(3):
+            assert load_library().chq_cycles(m._h, 2, ctypes.c_void_p(s.cuda_stream)) == 0
+    s.synchronize()
+    for x, y in ((a, b), (c, d)):
+        x.cycles(6)
+        assert x.clock() == y.clock()
+        bad = [f for f in FIELDS if not np.array_equal(x.get(f), y.get(f), equal_nan=True)]
+        x.close()
+        y.close()
+        assert not bad, bad
+
+
+@pytest.mark.parametrize("precision", [0, 1])
 def test_replayed_batches_equal_launches(precision):
     shapes = [(33, 30, 1), (20, 17, 11), (70, 1, 1), (41, 39, 40)]
     sets = [[mesh(s, precision, 2) for s in shapes] for _ in range(2)]
